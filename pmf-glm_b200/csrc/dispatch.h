@@ -18,6 +18,17 @@ struct StepKernelInfo {
 constexpr int kTileRows[] = {5, 8, 9, 13};
 constexpr int kNumTileRows = 4;
 
+// The instantiated (tile height, reconstruction) pairs, each compiled on its own (step_inst.cu).
+#define PMF_FOR_EACH_TILE(X) \
+  X(5, 0) X(5, 1) X(5, 2) X(8, 0) X(8, 1) X(8, 2) X(9, 0) X(9, 1) X(9, 2) X(13, 0) X(13, 1) X(13, 2)
+template <int TY, int RECON> StepKernelInfo step_kernel_info_of(int rsol, bool ct, bool comp, int src);
+template <int TY, int RECON> BatchKernel batch_kernel_of(int rsol, bool ct, bool comp);
+#define PMF_DECL(TY, RECON)                                                                            \
+  template <> StepKernelInfo step_kernel_info_of<TY, RECON>(int rsol, bool ct, bool comp, int src);    \
+  template <> BatchKernel batch_kernel_of<TY, RECON>(int rsol, bool ct, bool comp);
+PMF_FOR_EACH_TILE(PMF_DECL)
+#undef PMF_DECL
+
 // `src`: SRC_NONE, or a source-coupled step (SRC_DRAG, SRC_RAD; `comp` must be false).
 StepKernelInfo step_kernel_info(int ty, int recon, int rsol, bool ct, bool comp, int src = 0);
 // The many-box form of the same kernel (same shared memory and block size).

@@ -1,4 +1,4 @@
-// Lookup of the step-kernel instantiations for one tile height (included by step_ty*.cu).
+// Lookup of the step-kernel instantiations of one tile height and reconstruction (step_inst.cu).
 #pragma once
 #include "dispatch.h"
 #include "step_kernel.cuh"
@@ -31,15 +31,6 @@ BatchKernel pick_batch_rs(int rsol, bool ct, bool comp) {
   }
   return nullptr;
 }
-template <int TY>
-BatchKernel batch(int recon, int rsol, bool ct, bool comp) {
-  switch (recon) {
-    case RECON_PLM: return pick_batch_rs<TY, RECON_PLM>(rsol, ct, comp);
-    case RECON_PPM: return pick_batch_rs<TY, RECON_PPM>(rsol, ct, comp);
-    case RECON_PLM_MINMOD: return pick_batch_rs<TY, RECON_PLM_MINMOD>(rsol, ct, comp);
-  }
-  return nullptr;
-}
 template <int TY, int RECON>
 StepKernel pick_rs(int rsol, bool ct, bool comp, int src) {
   switch (rsol) {
@@ -48,16 +39,6 @@ StepKernel pick_rs(int rsol, bool ct, bool comp, int src) {
     case RS_LLF: return pick<TY, RECON, RS_LLF>(ct, comp, src);
   }
   return nullptr;
-}
-template <int TY>
-StepKernelInfo info(int recon, int rsol, bool ct, bool comp, int src) {
-  StepKernelInfo k{nullptr, StepSmem<TY>::BYTES, step_threads<TY>()};
-  switch (recon) {
-    case RECON_PLM: k.fn = pick_rs<TY, RECON_PLM>(rsol, ct, comp, src); break;
-    case RECON_PPM: k.fn = pick_rs<TY, RECON_PPM>(rsol, ct, comp, src); break;
-    case RECON_PLM_MINMOD: k.fn = pick_rs<TY, RECON_PLM_MINMOD>(rsol, ct, comp, src); break;
-  }
-  return k;
 }
 }  // namespace detail
 }  // namespace pmf
