@@ -38,60 +38,40 @@ struct HlldCensus {
   unsigned solves, ref_sides, rel_sides;
 };
 
-__device__ __forceinline__ F9 add9(const F9& a, const F9& b) {
-  F9 r;
-#pragma unroll
-  for (int i = 0; i < 9; ++i) r[i] = a[i] + b[i];
-  return r;
-}
-__device__ __forceinline__ F9 sub9(const F9& a, const F9& b) {
-  F9 r;
-#pragma unroll
-  for (int i = 0; i < 9; ++i) r[i] = a[i] - b[i];
-  return r;
-}
-__device__ __forceinline__ F9 neg9(const F9& a) {
-  F9 r;
-#pragma unroll
-  for (int i = 0; i < 9; ++i) r[i] = -a[i];
-  return r;
-}
-
 // ---- packed FP32 pairs (sm_100 FFMA2 / FMUL2 / FADD2): two independent evaluations of the
 // same expression in one instruction, each lane rounded exactly as the scalar operation ----
 __device__ __forceinline__ float2 p2(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ float2 pb(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-// a*b - c*d per lane
-__device__ __forceinline__ float2 msub2(float2 a, float2 b, float2 c, float2 d) {
-  return fma2(a, b, make_float2(-(c.x * d.x), -(c.y * d.y)));
-}
 struct P9 {
   float2 v[9];
   __device__ __forceinline__ float2& operator[](int i) { return v[i]; }
   __device__ __forceinline__ const float2& operator[](int i) const { return v[i]; }
 };
 
+// Products that meet an add are written as explicit fused multiply-adds or explicitly rounded
+// products here and in the solvers below: left to the compiler, which of them fuse depends on the
+// instantiation, and the step's instantiations are to give the same bits.
+
 // conserved -> primitive with density and pressure floors (glm_physics.jl:11-18)
 __device__ __forceinline__ F9 cons2prim(const F9& c, float g, float smallr, float pfl) {
-  float rho = fmaxf(c[0], smallr);
-  float ir = 1.0f / rho;
-  float vx = c[1] * ir, vy = c[2] * ir, vz = c[3] * ir;
-  float bx = c[5], by = c[6], bz = c[7];
-  float ekin = 0.5f * (c[1] * c[1] + c[2] * c[2] + c[3] * c[3]) * ir;
-  float emag = 0.5f * (bx * bx + by * by + bz * bz);
-  float p = fmaxf((g - 1.0f) * (c[4] - ekin - emag), pfl);
-  return F9{{rho, vx, vy, vz, p, bx, by, bz, c[8]}};
+  const float rho = fmaxf(c[0], smallr);
+  const float ir = 1.0f / rho;
+  const float m2 = fmaf(c[3], c[3], fmaf(c[2], c[2], c[1] * c[1]));
+  const float b2 = fmaf(c[7], c[7], fmaf(c[6], c[6], c[5] * c[5]));
+  const float ei = fmaf(-0.5f, b2, fmaf(-0.5f * m2, ir, c[4]));
+  const float p = fmaxf((g - 1.0f) * ei, pfl);
+  return F9{{rho, __fmul_rn(c[1], ir), __fmul_rn(c[2], ir), __fmul_rn(c[3], ir), p, c[5], c[6], c[7], c[8]}};
 }
 
 // primitive -> conserved (glm_physics.jl:19-23)
 __device__ __forceinline__ F9 prim2cons(const F9& q, float g) {
-  float rho = q[0], vx = q[1], vy = q[2], vz = q[3], p = q[4], bx = q[5], by = q[6], bz = q[7];
-  float E = p / (g - 1.0f) + 0.5f * rho * (vx * vx + vy * vy + vz * vz) + 0.5f * (bx * bx + by * by + bz * bz);
-  return F9{{rho, rho * vx, rho * vy, rho * vz, E, bx, by, bz, q[8]}};
+  const float rho = q[0], vx = q[1], vy = q[2], vz = q[3], bx = q[5], by = q[6], bz = q[7];
+  const float v2 = fmaf(vz, vz, fmaf(vy, vy, vx * vx)), b2 = fmaf(bz, bz, fmaf(by, by, bx * bx));
+  const float E = fmaf(0.5f, b2, fmaf(0.5f * rho, v2, q[4] * (1.0f / (g - 1.0f))));
+  return F9{{rho, __fmul_rn(rho, vx), __fmul_rn(rho, vy), __fmul_rn(rho, vz), E, bx, by, bz, q[8]}};
 }
 
 // fast magnetosonic speed along the normal with normal field bn (glm_physics.jl:24-27)
@@ -185,26 +165,15 @@ __device__ __forceinline__ float min_xorsign_abs(float a, float b) {
 __device__ __forceinline__ float half_moncen(float dl, float dr, float q) {
   return min_xorsign_abs(fmaxf(min_xorsign_abs(dl, dr), 0.0f), q);
 }
-// Two fields at once: the differences and the quarter sum as packed pairs (each lane rounded as
-// the scalar operation), the limiter per lane.
-__device__ __forceinline__ float2 half_moncen2(float2 mm, float2 m0, float2 mp) {
-  const float2 dl = sub2(m0, mm), dr = sub2(mp, m0);
-  const float2 q = mul2(pb(0.25f), add2(dl, dr));
-  return make_float2(half_moncen(dl.x, dr.x, q.x), half_moncen(dl.y, dr.y, q.y));
-}
-
 template <int RECON>
 __device__ __forceinline__ Offsets<RECON> recon(const F9& mm, const F9& m0, const F9& mp) {
   Offsets<RECON> o;
   if constexpr (RECON == RECON_PLM) {
 #pragma unroll
-    for (int i = 0; i < 8; i += 2) {
-      const float2 h = half_moncen2(p2(mm[i], mm[i + 1]), p2(m0[i], m0[i + 1]), p2(mp[i], mp[i + 1]));
-      o.dR[i] = h.x;
-      o.dR[i + 1] = h.y;
+    for (int i = 0; i < 9; ++i) {
+      const float dl = m0[i] - mm[i], dr = mp[i] - m0[i];
+      o.dR[i] = half_moncen(dl, dr, 0.25f * (dl + dr));
     }
-    const float dl = m0[8] - mm[8], dr = mp[8] - m0[8];
-    o.dR[8] = half_moncen(dl, dr, 0.25f * (dl + dr));
   } else if constexpr (RECON == RECON_PLM_MINMOD) {
 #pragma unroll
     for (int i = 0; i < 9; ++i) o.dR[i] = 0.5f * minmod(m0[i] - mm[i], mp[i] - m0[i]);
@@ -232,49 +201,59 @@ template <int RECON> __device__ __forceinline__ F9 face_hi(const F9& mh, const O
   return r;
 }
 
-// x-normal flux of two primitive states at once (lane x and lane y), glm_physics.jl:28-34.
-__device__ __forceinline__ P9 phys_flux_x2(const P9& q, float g) {
-  const float2 rho = q[0], vx = q[1], vy = q[2], vz = q[3], p = q[4], bx = q[5], by = q[6], bz = q[7];
-  const float2 b2 = fma2(bz, bz, fma2(by, by, mul2(bx, bx)));
-  const float2 half = pb(0.5f);
-  const float2 ptot = fma2(half, b2, p);
-  const float2 v2 = fma2(vz, vz, fma2(vy, vy, mul2(vx, vx)));
-  const float ig = 1.0f / (g - 1.0f);
-  const float2 E = fma2(half, b2, fma2(mul2(half, rho), v2, mul2(p, pb(ig))));
-  const float2 vb = fma2(vz, bz, fma2(vy, by, mul2(vx, bx)));
-  const float2 m = mul2(rho, vx);
-  P9 f;
-  f[0] = m;
-  f[1] = sub2(fma2(m, vx, ptot), mul2(bx, bx));
-  f[2] = sub2(mul2(m, vy), mul2(bx, by));
-  f[3] = sub2(mul2(m, vz), mul2(bx, bz));
-  f[4] = sub2(mul2(add2(E, ptot), vx), mul2(bx, vb));
-  f[5] = pb(0.0f);
-  f[6] = sub2(mul2(vx, by), mul2(vy, bx));
-  f[7] = sub2(mul2(vx, bz), mul2(vz, bx));
-  f[8] = pb(0.0f);
-  return f;
-}
-
-// flux difference F(m0 + dR) - F(m0 + dL) along axis D (one term of the Hancock predictor,
-// glm_physics.jl:225-231); the flux of the two face states is evaluated as one packed pair (the
-// states themselves are formed by scalar adds, which write the pair's registers directly)
-template <int D, int RECON>
-__device__ __forceinline__ F9 hancock_term(const F9& m0, const Offsets<RECON>& o, float g) {
+// One term of the Hancock predictor (glm_physics.jl:225-231): the x-normal fluxes (D-normal after
+// the axis permutation) of the two face states m0 + dR (lane x) and m0 + dL (lane y), added to the
+// packed sums `acc` (global component order; FIRST: the sums start here). The sums enter the
+// multiply-adds that form each flux, so adding a direction costs nothing beyond its flux. A packed
+// subtraction is avoided throughout: negating both lanes of an operand costs two instructions
+// beside the packed one (measured 4 issue cycles against 2), so the normal field is negated once.
+template <int D, int RECON, bool FIRST>
+__device__ __forceinline__ void hancock_term(P9& acc, const F9& m0, const Offsets<RECON>& o, float g) {
   // global -> D-normal component order, as rot_to<D>
   constexpr int perm[3][9] = {{0, 1, 2, 3, 4, 5, 6, 7, 8}, {0, 2, 3, 1, 4, 6, 7, 5, 8}, {0, 3, 1, 2, 4, 7, 5, 6, 8}};
   P9 q;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) {
+  for (int i = 0; i < 8; ++i) {
     const int j = perm[D][i];
     q[i] = make_float2(m0[j] + o.dR[j], m0[j] + o.l(j));
   }
-  const P9 f = phys_flux_x2(q, g);
-  F9 d;
-  // back to the global order (rot_back<D>) while taking the difference of the two lanes
-#pragma unroll
-  for (int i = 0; i < 9; ++i) d[perm[D][i]] = f[i].x - f[i].y;
-  return d;
+  const float2 rho = q[0], vx = q[1], vy = q[2], vz = q[3], p = q[4], bx = q[5], by = q[6], bz = q[7];
+  const float2 half = pb(0.5f);
+  const float2 nbx = mul2(bx, pb(-1.0f));
+  const float2 b2 = fma2(bz, bz, fma2(by, by, mul2(bx, bx)));
+  const float2 v2 = fma2(vz, vz, fma2(vy, vy, mul2(vx, vx)));
+  const float2 vb = fma2(vz, bz, fma2(vy, by, mul2(vx, bx)));
+  const float2 h = fma2(mul2(half, rho), v2, fma2(p, pb(1.0f + 1.0f / (g - 1.0f)), b2));  // E + ptot
+  const float2 m = mul2(rho, vx);
+  // a * b added to component c
+  auto mad = [&](int c, float2 a, float2 b) { acc[c] = FIRST ? mul2(a, b) : fma2(a, b, acc[c]); };
+  constexpr int M = perm[D][1], V = perm[D][2], W = perm[D][3], BV = perm[D][6], BW = perm[D][7];
+  const float2 ptm = fma2(m, vx, fma2(half, b2, p));
+  if (FIRST) {
+    acc[0] = m;
+    acc[M] = fma2(nbx, bx, ptm);
+  } else {
+    acc[0] = add2(acc[0], m);
+    acc[M] = add2(acc[M], fma2(nbx, bx, ptm));
+  }
+  mad(V, m, vy);
+  acc[V] = fma2(nbx, by, acc[V]);
+  mad(W, m, vz);
+  acc[W] = fma2(nbx, bz, acc[W]);
+  mad(4, h, vx);
+  acc[4] = fma2(nbx, vb, acc[4]);
+  if (D == 0) {  // By and Bz start with x, Bx with y
+    acc[BV] = mul2(vx, by);
+    acc[BW] = mul2(vx, bz);
+  } else if (D == 1) {  // normal By: transverse (Bz, Bx)
+    acc[BV] = fma2(vx, by, acc[BV]);
+    acc[BW] = mul2(vx, bz);
+  } else {
+    acc[BV] = fma2(vx, by, acc[BV]);
+    acc[BW] = fma2(vx, bz, acc[BW]);
+  }
+  acc[BV] = fma2(nbx, vy, acc[BV]);
+  acc[BW] = fma2(nbx, vz, acc[BW]);
 }
 
 // ---- Riemann solvers in the face-normal frame (x-normal after rot_to) -----------------
@@ -303,56 +282,66 @@ __device__ __forceinline__ F9 hll_x(const F9& L, const F9& R, float g, float bn,
   f[8] = fpsi;
   return f;
 }
-// HLLD, Miyoshi & Kusano 2005 (glm_physics.jl:255-307). The left and right halves of the
-// solver are the same algebra on the two states, so they run as packed pairs (lane x = L,
-// lane y = R); the scalar parts are the wave speeds, the contact speed and the doubly-starred
-// state, which mix both sides.
+// HLLD, Miyoshi & Kusano 2005 (glm_physics.jl:255-307). The parts that are the same algebra on the
+// two states run as packed pairs (lane x = L, lane y = R).
+//
+// The reference forms the single-star states of both sides, v* = v - bn b x and b* = (1 + d(S-u) x) b
+// with x = (S_M - u) / denK, denK = d(S-u)(S-S_M) - bn^2, the double-star state from them, and the
+// flux F_K + S_K (U*_K - U_K) (outer region) or F_K + S*_K U** - (S*_K - S_K) U*_K - S_K U_K (inner
+// region) of the side K that the contact leans to. Here the same flux is reduced with
+//   S_K - S*_K = denK / (|d(S-u)| + sqrt(d*) |bn|),   D = |S - S_M| + |S* - S_M|,
+// so that only what the selected region needs is formed and the inner region has no 1/denK:
+//   b' = b (1 + s r), r = (S_M - u) / D (s = -1 left, +1 right) takes the place of b* in the
+//   double-star averages (v is unchanged there), and with m = d* S_M, t = 0 (outer) or S*_K (inner),
+//   y = S_K d* x (outer) or s r (inner):
+//   F(mass) = m, F(normal) = m S_M + ptot* - bn^2, F(v) = m v + d* t (v** - v) - bn b (1 + y),
+//   F(b) = b (u + (S_K - S_M) y) + t (b** - b) - bn v,
+//   F(E) = S_M (G + S_K ptot*) / (S_K - S_M) + c w - s sqrt(d*) sgn(bn) t w**,
+// G = (S-u) E - ptot u + bn v.B, w = v*.B*, w** = v**.B**, c = -S_K bn / (S_K - S_M) (outer) or
+// sgn(bn) S_M denK / (sqrt(d*) D (S_K - S_M)) (inner). Near R-degenerate faces, where denK is the
+// rounding residue of two terms of size bn^2, the inner flux keeps FP32 accuracy.
+// The step is bounded by instruction issue: with this form, the predictor's sums in multiply-adds
+// and the vectorised tile edges the 256^3 GLM step executes 58 instead of 72 warp instructions
+// per cell (1.77 -> 1.54 ms; constrained transport 2.29 -> 2.05 ms).
 __device__ __forceinline__ F9 hlld_x(const F9& L, const F9& R, float g, float bn, float fbn, float fpsi,
                                      float dtol_rel, HlldCensus* cen = nullptr) {
   const float2 d = p2(L[0], R[0]), u = p2(L[1], R[1]), v = p2(L[2], R[2]), w = p2(L[3], R[3]);
   const float2 p = p2(L[4], R[4]), by = p2(L[6], R[6]), bz = p2(L[7], R[7]);
   const float2 half = pb(0.5f);
   const float bn2 = bn * bn;
+  const float2 nbn2 = pb(-bn2);
   const float2 b2 = fma2(bz, bz, fma2(by, by, pb(bn2)));
   const float2 pt = fma2(half, b2, p);
-  const float ig = 1.0f / (g - 1.0f);
-  const float2 E = fma2(half, b2, fma2(mul2(half, d), fma2(w, w, fma2(v, v, mul2(u, u))), mul2(p, pb(ig))));
   // fast speeds (glm_physics.jl:24-27) with the normal field bn
   const float2 id = p2(1.0f / L[0], 1.0f / R[0]);
   const float2 c2 = mul2(mul2(pb(g), p), id);
-  const float2 bb = mul2(b2, id);
-  const float2 d2 = mul2(half, add2(bb, c2));
-  const float2 disc = sub2(mul2(d2, d2), mul2(mul2(c2, pb(bn2)), id));
+  const float2 d2 = mul2(half, fma2(b2, id, c2));
+  const float2 disc = fma2(d2, d2, mul2(mul2(c2, nbn2), id));
   const float2 in = add2(d2, p2(sqrtf(fmaxf(disc.x, 0.0f)), sqrtf(fmaxf(disc.y, 0.0f))));
-  const float cfL = sqrtf(in.x), cfR = sqrtf(in.y);
-  const float cf = fmaxf(cfL, cfR);
+  const float cf = sqrtf(fmaxf(in.x, in.y));
   const float SL = fminf(fminf(u.x, u.y) - cf, 0.0f);
   const float SR = fmaxf(fmaxf(u.x, u.y) + cf, 0.0f);
   const float2 S = p2(SL, SR);
-  const float2 Su = sub2(S, u);         // S - u per side
-  const float2 dSu = mul2(Su, d);       // d (S - u)
-  const float den = dSu.y - dSu.x;
-  const float2 dSuu = mul2(dSu, u);
-  const float SM = ((dSuu.y - dSuu.x) - pt.y + pt.x) / den;
-  const float pts = ((dSu.y * pt.x - dSu.x * pt.y) + d.x * d.y * Su.y * Su.x * (u.y - u.x)) / den;
-  const float2 SSM = sub2(S, pb(SM));   // S - SM per side
-  const float2 ds = mul2(dSu, p2(1.0f / SSM.x, 1.0f / SSM.y));
+  const float2 dSu = mul2(p2(SL - u.x, SR - u.y), d);  // d (S - u) per side
+  const float iden = 1.0f / (dSu.y - dSu.x);
+  const float SM = __fmul_rn(fmaf(dSu.y, u.y, pt.x) - fmaf(dSu.x, u.x, pt.y), iden);
+  const float pts = __fmul_rn(fmaf(dSu.y, fmaf(dSu.x, u.y - u.x, pt.x), -dSu.x * pt.y), iden);
+  const float2 SSM = add2(S, pb(-SM));  // S - SM per side
+  const float2 iSSM = p2(1.0f / SSM.x, 1.0f / SSM.y);
+  const float2 ds = mul2(dSu, iSSM);
   const float dLs = fmaxf(ds.x, 1e-12f), dRs = fmaxf(ds.y, 1e-12f);
-  const float2 dst = p2(dLs, dRs);
-  const float sqL = sqrtf(dLs), sqR = sqrtf(dRs);
+  const float irL = rsqrtf(dLs), irR = rsqrtf(dRs);
+  const float sqL = __fmul_rn(dLs, irL), sqR = __fmul_rn(dRs, irR);
   const float abn = fabsf(bn);
-  const float SLs = SM - abn / sqL, SRs = SM + abn / sqR;
-  // single-starred transverse states of both sides (glm_physics.jl:255-263)
-  const float2 denK = fma2(dSu, SSM, pb(-bn2));
-  const float2 nK = fma2(dSu, Su, pb(-bn2));       // d (S - u)^2 - bn^2
-  const float2 iK = p2(1.0f / denK.x, 1.0f / denK.y);
-  const float2 fac = mul2(mul2(pb(bn), sub2(pb(SM), u)), iK);
-  const float2 rK = mul2(nK, iK);
+  const float SLs = fmaf(-abn, irL, SM), SRs = fmaf(abn, irR, SM);
+  const float iDL = 1.0f / fmaf(abn, irL, fabsf(SSM.x)), iDR = 1.0f / fmaf(abn, irR, fabsf(SSM.y));
+  float2 r = p2((u.x - SM) * iDL, (SM - u.y) * iDR);  // s r per side
   // Degenerate star state (the fast and Alfven speeds coincide). The reference tests
   // |denK| < 1e-12 (dtol_rel = 0), which is below the FP32 rounding of denK = d(S-u)(S-SM) - bn^2
-  // (a difference of two terms of size bn^2): a 1-ulp residue then makes the single-star states
-  // ~1/denK and the fan flux depends on a cancellation (S*_L - S_L) * U*_L. The relative mode
-  // (dtol_rel = 1e-5) sends faces with |denK| within 1e-5 bn^2 of zero to the degenerate branch.
+  // (a difference of two terms of size bn^2). The relative mode (dtol_rel = 1e-5) sends faces with
+  // |denK| within 1e-5 bn^2 of zero to the degenerate branch, whose transverse state is the
+  // unmodified one (v* = v, b* = b: x = r = 0).
+  const float2 denK = fma2(dSu, SSM, nbn2);
   const float dtol = fmaxf(1e-12f, dtol_rel * bn2);
   const bool degL = fabsf(denK.x) < dtol, degR = fabsf(denK.y) < dtol;
   if (cen != nullptr) {
@@ -361,46 +350,49 @@ __device__ __forceinline__ F9 hlld_x(const F9& L, const F9& R, float g, float bn
     cen->ref_sides += (aL < 1e-12f ? 1u : 0u) + (aR < 1e-12f ? 1u : 0u);
     cen->rel_sides += (aL >= 1e-12f && aL < t5 ? 1u : 0u) + (aR >= 1e-12f && aR < t5 ? 1u : 0u);
   }
-  float2 vs = sub2(v, mul2(by, fac)), ws = sub2(w, mul2(bz, fac));
-  float2 bys = mul2(by, rK), bzs = mul2(bz, rK);
-  if (degL) { vs.x = v.x; ws.x = w.x; bys.x = by.x; bzs.x = bz.x; }
-  if (degR) { vs.y = v.y; ws.y = w.y; bys.y = by.y; bzs.y = bz.y; }
-  const float2 vdb = fma2(w, bz, fma2(v, by, mul2(u, pb(bn))));
-  const float2 vdbs = fma2(ws, bzs, fma2(vs, bys, pb(SM * bn)));
-  // E* = ((S - u) E - pt u + pts SM + bn (v.b - v*.b*)) / (S - SM)
-  const float2 Enum = fma2(pb(bn), sub2(vdb, vdbs), add2(sub2(mul2(Su, E), mul2(pt, u)), pb(pts * SM)));
-  const float2 Es = mul2(Enum, p2(1.0f / SSM.x, 1.0f / SSM.y));
-  const float sgn = bn >= 0.0f ? 1.0f : -1.0f;
-  const float invsum = 1.0f / (sqL + sqR);
-  const float vyss = (sqL * vs.x + sqR * vs.y + (bys.y - bys.x) * sgn) * invsum;
-  const float vzss = (sqL * ws.x + sqR * ws.y + (bzs.y - bzs.x) * sgn) * invsum;
-  const float byss = (sqL * bys.y + sqR * bys.x + sqL * sqR * (vs.y - vs.x) * sgn) * invsum;
-  const float bzss = (sqL * bzs.y + sqR * bzs.x + sqL * sqR * (ws.y - ws.x) * sgn) * invsum;
-  const float vdbss = SM * bn + vyss * byss + vzss * bzss;
-  // E** = E* -+ sqrt(d*) (v*.b* - v**.b**) sgn
-  const float2 Ess = fma2(mul2(p2(-sqL, sqR), pb(sgn)), sub2(vdbs, pb(vdbss)), Es);
-  // only the selected fan state is assembled: the four branches of glm_physics.jl:297-305
-  F9 f;
+  if (degL) r.x = 0.0f;
+  if (degR) r.y = 0.0f;
+  // double-star transverse state, with the density-root weights wa, wb = 1 - wa
+  const float2 bye = fma2(by, r, by), bze = fma2(bz, r, bz);
+  const float inv = 1.0f / (sqL + sqR);
+  const float wb = sqR * inv, wa = sqL * inv;
+  const float c = copysignf(inv, bn), e = sqL * sqR * c;
+  const float dv = v.y - v.x, dw = w.y - w.x, dby = bye.y - bye.x, dbz = bze.y - bze.x;
+  const float vyss = fmaf(c, dby, fmaf(wb, dv, v.x)), vzss = fmaf(c, dbz, fmaf(wb, dw, w.x));
+  const float byss = fmaf(e, dv, fmaf(wa, dby, bye.x)), bzss = fmaf(e, dw, fmaf(wa, dbz, bze.x));
+  const float SMbn = SM * bn;
+  const float wss = fmaf(vzss, bzss, fmaf(vyss, byss, SMbn));
+  // the side the contact leans to
   const bool left = SM >= 0.0f;
   const float dK = left ? d.x : d.y, uK = left ? u.x : u.y, vK = left ? v.x : v.y, wK = left ? w.x : w.y;
-  const float pK = left ? p.x : p.y, byK = left ? by.x : by.y, bzK = left ? bz.x : bz.y;
-  const float EK = left ? E.x : E.y, SK = left ? SL : SR, dKs = left ? dLs : dRs;
-  const float vKs = left ? vs.x : vs.y, wKs = left ? ws.x : ws.y, byKs = left ? bys.x : bys.y;
-  const float bzKs = left ? bzs.x : bzs.y, EKs = left ? Es.x : Es.y, EKss = left ? Ess.x : Ess.y;
-  const float SKs = left ? SLs : SRs;
+  const float pK = left ? p.x : p.y, byK = left ? by.x : by.y, bzK = left ? bz.x : bz.y, SK = left ? SL : SR;
+  const float iSSMK = left ? iSSM.x : iSSM.y, dKs = left ? dLs : dRs, irK = left ? irL : irR;
+  const float iDK = left ? iDL : iDR, rK = left ? r.x : r.y, SKs = left ? SLs : SRs;
+  const float denKK = left ? denK.x : denK.y;
+  const bool degK = left ? degL : degR;
   const bool outer = left ? (SLs >= 0.0f) : (SRs < 0.0f);
-  const F9 FK = phys_flux_x(F9{{dK, uK, vK, wK, pK, bn, byK, bzK, 0.0f}}, g);
-  const float UK[8] = {dK, dK * uK, dK * vK, dK * wK, EK, bn, byK, bzK};
-  const float UKs[8] = {dKs, dKs * SM, dKs * vKs, dKs * wKs, EKs, bn, byKs, bzKs};
-  if (outer) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = FK[i] + SK * (UKs[i] - UK[i]);
-  } else {
-    const float UKss[8] = {dKs, dKs * SM, dKs * vyss, dKs * vzss, EKss, bn, byss, bzss};
-#pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = FK[i] + SKs * UKss[i] - (SKs - SK) * UKs[i] - SK * UK[i];
-  }
+  const float SuK = SK - uK, dSuK = dK * SuK, SSMK = SK - SM;
+  const float bt2 = fmaf(bzK, bzK, byK * byK), vbt = fmaf(wK, bzK, vK * byK);
+  const float b2K = fmaf(bn, bn, bt2);
+  const float EK = fmaf(0.5f * dK, fmaf(wK, wK, fmaf(vK, vK, uK * uK)), fmaf(pK, 1.0f / (g - 1.0f), 0.5f * b2K));
+  const float G = fmaf(bn, fmaf(uK, bn, vbt), fmaf(SuK, EK, -fmaf(0.5f, b2K, pK) * uK));
+  const float x = degK ? 0.0f : (SM - uK) * (1.0f / denKK);
+  const float ws = fmaf(fmaf(dSuK, x, 1.0f), fmaf(-bn * x, bt2, vbt), SMbn);
+  const float sgn = copysignf(1.0f, bn);
+  const float t = outer ? 0.0f : SKs;
+  const float y = outer ? SK * dKs * x : rK;
+  const float cw = outer ? -SK * bn : sgn * SM * (denKK * (irK * iDK));
+  const float sqK = sgn * (left ? -sqL : sqR);
+  const float dt_ = dKs * t, by1 = fmaf(bn, y, bn), bu = fmaf(SSMK, y, uK);
+  F9 f;
+  f[0] = __fmul_rn(dKs, SM);
+  f[1] = fmaf(f[0], SM, fmaf(-bn, bn, pts));
+  f[2] = fmaf(dt_, vyss - vK, fmaf(f[0], vK, -by1 * byK));
+  f[3] = fmaf(dt_, vzss - wK, fmaf(f[0], wK, -by1 * bzK));
+  f[4] = fmaf(iSSMK, fmaf(SM, fmaf(SK, pts, G), cw * ws), -sqK * t * wss);
   f[5] = fbn;
+  f[6] = fmaf(t, byss - byK, fmaf(bu, byK, -bn * vK));
+  f[7] = fmaf(t, bzss - bzK, fmaf(bu, bzK, -bn * wK));
   f[8] = fpsi;
   return f;
 }
@@ -417,9 +409,9 @@ __device__ __forceinline__ F9 riemann_glm(const F9& Lq, const F9& Rq, float ch, 
   F9 L = rot_to<D>(Lq), R = rot_to<D>(Rq);
   L[0] = fmaxf(L[0], P.smallr); L[4] = fmaxf(L[4], P.pfl);
   R[0] = fmaxf(R[0], P.smallr); R[4] = fmaxf(R[4], P.pfl);
-  float bns = 0.5f * (L[5] + R[5]) - 0.5f * (R[8] - L[8]) * ich;
-  float psis = 0.5f * (L[8] + R[8]) - 0.5f * ch * (R[5] - L[5]);
-  float fbn = psis, fpsi = ch * ch * bns;
+  float bns = fmaf(-0.5f * (R[8] - L[8]), ich, 0.5f * (L[5] + R[5]));
+  float psis = fmaf(-0.5f * ch, R[5] - L[5], 0.5f * (L[8] + R[8]));
+  float fbn = psis, fpsi = __fmul_rn(ch * ch, bns);
   L[5] = bns; R[5] = bns;
   F9 f;
   if constexpr (RSOL == RS_LLF) {

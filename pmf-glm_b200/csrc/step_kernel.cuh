@@ -119,7 +119,7 @@ struct StepSmem {
   static constexpr int YB = (TY + 1) * G9;          // y-face states / fluxes
   static constexpr int ZC = TY * 3 * G9;            // per owned thread: upper z state, lower z flux, x/y divergence
   static constexpr int YL = (TY + 1) * G9;          // lower y state of rows 1..TY+1, parked
-  static constexpr int XB = TY * 9;                 // one x-face state or flux per owned row
+  static constexpr int XB = TY * 12;                // one x-face state or flux per owned row
   static constexpr int NL = 96;                     // loader threads: warps 0, TY+1 and the halo warp
   static constexpr int KL = (PW + NL - 1) / NL;     // staged entries per loader thread
   static constexpr int SI = 2 * KL * NL;            // per loader: source (x, y) offset; ring cell and flip bits
@@ -149,6 +149,21 @@ template <int NC> __device__ __forceinline__ F9 ld9p(const float* pl, int c) {
   const float4 a = reinterpret_cast<const float4*>(pl)[c];
   const float4 b = reinterpret_cast<const float4*>(pl)[NC + c];
   return F9{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, pl[8 * NC + c]}};
+}
+
+// Nine values of one tile-edge state or flux in 12 floats: three vector instructions, which one
+// lane of a row warp (or the halo warp's lanes) executes while the other lanes wait. As nine
+// predicated scalar accesses at each of the five places these took 4 % of the step (256^3 GLM
+// step 1.62 -> 1.545 ms).
+__device__ __forceinline__ void st9x(float* g, const F9& v) {
+  reinterpret_cast<float4*>(g)[0] = make_float4(v[0], v[1], v[2], v[3]);
+  reinterpret_cast<float4*>(g)[1] = make_float4(v[4], v[5], v[6], v[7]);
+  g[8] = v[8];
+}
+__device__ __forceinline__ F9 ld9x(const float* g) {
+  const float4 a = reinterpret_cast<const float4*>(g)[0];
+  const float4 b = reinterpret_cast<const float4*>(g)[1];
+  return F9{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, g[8]}};
 }
 
 __device__ __forceinline__ void cp_async4(float* smem_dst, const float* gsrc) {
@@ -181,9 +196,9 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
   float* fybuf = ybuf + S::YB;     // [row-1] flux through the lower y face of rows 1..TY+1
   float* zcarry = fybuf + S::YB;   // [row][3] upper z state, lower z flux, x/y divergence of p-1
   float* ylow = zcarry + S::ZC;    // [row-1] lower y state of rows 1..TY+1
-  float* xleft = ylow + S::YL;     // [row][9] upper x state of the left halo cell
-  float* xright = xleft + S::XB;   // [row][9] upper x state of lane 31
-  float* fxright = xright + S::XB; // [row][9] flux through the face above lane 31
+  float* xleft = ylow + S::YL;     // [row][12] upper x state of the left halo cell
+  float* xright = xleft + S::XB;   // [row][12] upper x state of lane 31
+  float* fxright = xright + S::XB; // [row][12] flux through the face above lane 31
   int* sidx = reinterpret_cast<int*>(fxright + S::XB);  // [KL][2][NL] staging map of this segment
 
   const int tid = threadIdx.x;
@@ -413,8 +428,11 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
     F9 un;
     float d[9];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) d[i] = dtdx * (dxy[i] + (flo[i] - fhi[i]));
-    un[0] = u0[0] + d[0];
+    for (int i = 0; i < 9; ++i) {
+      const float div = dxy[i] + (flo[i] - fhi[i]);
+      d[i] = dtdx * div;
+      un[i] = fmaf(dtdx, div, u0[i]);
+    }
     if constexpr (COMP) {
 #pragma unroll
       for (int i = 1; i <= NR; ++i) {
@@ -422,13 +440,6 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
         un[i] = comp_add(u0[i], d[i], r);
         a.resid[i - 1][c] = r;
       }
-      if constexpr (CT) {
-#pragma unroll
-        for (int i = NR + 1; i <= 7; ++i) un[i] = u0[i] + d[i];
-      }
-    } else {
-#pragma unroll
-      for (int i = 1; i <= 7; ++i) un[i] = u0[i] + d[i];
     }
     if constexpr (RAD) {
       // radiation-coupled update (integrator_cube.jl:85-106,412-436; integrator_ref.jl:140-156):
@@ -449,7 +460,6 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
           cr[(size_t)i * n + cc] = r;
         }
       }
-      un[8] = u0[8] + d[8];
       const bool bad = (fl & RAD_CHECK) && inadmissible_cell(un, P);
       drag_correct_cell(u0, un, a.drag, P.smallr, (fl & RAD_TRACK_ENERGY) ? &rE : nullptr);
       if (fl & RAD_TRACK_ENERGY) cr[8 * n + cc] = rE;
@@ -459,7 +469,7 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
       // which CT later replaces by the face average); integrator_ref.jl:155-156
       drag_correct_cell(u0, un, a.drag, P.smallr);
     }
-    un[8] = CT ? 0.0f : (u0[8] + d[8]) * decay;
+    un[8] = CT ? 0.0f : un[8] * decay;
 #pragma unroll
     for (int f = 0; f < 9; ++f) {
       if (CT && f >= 5 && f <= 7) continue;  // cell B comes from the face average
@@ -484,14 +494,13 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
     // x/y flux divergence of plane p-1 for the owned rows, parked for its update in the z-solve
     // of this pass (the face above lane 31 comes from the halo warp)
     if (row_own && p > z0) {
-      F9 dxy;
+      F9 dxy, fxh;
       const F9 fyl = ld9g(fybuf + (w - 1) * S::G9, lane), fyh = ld9g(fybuf + w * S::G9, lane);
 #pragma unroll
-      for (int i = 0; i < 9; ++i) {
-        const float dn = __shfl_down_sync(0xffffffffu, Fx[i], 1);
-        const float fxh = lane == TILE_X - 1 ? fxright[(w - 1) * 9 + i] : dn;
-        dxy[i] = (Fx[i] - fxh) + (fyl[i] - fyh[i]);
-      }
+      for (int i = 0; i < 9; ++i) fxh[i] = __shfl_down_sync(0xffffffffu, Fx[i], 1);
+      if (lane == TILE_X - 1) fxh = ld9x(fxright + (w - 1) * 12);
+#pragma unroll
+      for (int i = 0; i < 9; ++i) dxy[i] = (Fx[i] - fxh[i]) + (fyl[i] - fyh[i]);
       zc_store(ZC_DIV, dxy);
     }
     const bool mid = p >= z0 && p < z1;  // an owned plane of this chunk
@@ -535,13 +544,15 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
     }
     {
       const F9 u0 = prim2cons(m0, g);
-      F9 acc = hancock_term<0, RECON>(m0, ox, g);
-      acc = add9(acc, hancock_term<1, RECON>(m0, oy, g));
-      acc = add9(acc, hancock_term<2, RECON>(m0, oz, g));
+      P9 acc;
+      hancock_term<0, RECON, true>(acc, m0, ox, g);
+      hancock_term<1, RECON, false>(acc, m0, oy, g);
+      hancock_term<2, RECON, false>(acc, m0, oz, g);
       const float h = 0.5f * dtdx;
       F9 uh;
 #pragma unroll
-      for (int i = 0; i < 9; ++i) uh[i] = u0[i] - h * acc[i];
+      for (int i = 0; i < 8; ++i) uh[i] = fmaf(-h, acc[i].x - acc[i].y, u0[i]);
+      uh[8] = u0[8];
       mh = cons2prim(uh, g, P.smallr, P.pfl);
     }
     // drag: face states and the CT cell EMF see the drag-propagated velocity
@@ -579,13 +590,11 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
     // x-face states at the tile edges go through shared memory
     if (mid && row_own && lane == TILE_X - 1) {
       const F9 xR = face_hi<RECON>(mh, ox);
-#pragma unroll
-      for (int i = 0; i < 9; ++i) xright[(w - 1) * 9 + i] = xR[i];
+      st9x(xright + (w - 1) * 12, xR);
     }
     if (mid && halo_act && hside == 0) {
       const F9 xR = face_hi<RECON>(mh, ox);
-#pragma unroll
-      for (int i = 0; i < 9; ++i) xleft[hrow * 9 + i] = xR[i];
+      st9x(xleft + hrow * 12, xR);
     }
     if (row_own) {
       // ---- z-face p-1/2: left = carried upper z state of p-1, right = lower z state of p --
@@ -640,18 +649,12 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
         for (int i = 0; i < 9; ++i) L[i] = __shfl_up_sync(0xffffffffu, xR[i], 1);
       }
       if (row_own || (halo_act && hside == 1)) {
-#pragma unroll
-        for (int i = 0; i < 9; ++i)
-          if (halo_warp) L[i] = xright[hrow * 9 + i];
-          else if (lane == 0) L[i] = xleft[(w - 1) * 9 + i];
+        if (halo_warp || lane == 0) L = ld9x(halo_warp ? xright + hrow * 12 : xleft + (w - 1) * 12);
         if constexpr (CT) {
           L[5] = bnx; R[5] = bnx;
         }
         Fx = riemann<0, RSOL, CT>(L, R, ch, ich, P, own ? &cz : nullptr, masked && (m_c || mask_at(p, rad_xm)));
-        if (halo_warp) {
-#pragma unroll
-          for (int i = 0; i < 9; ++i) fxright[hrow * 9 + i] = Fx[i];
-        }
+        if (halo_warp) st9x(fxright + hrow * 12, Fx);
         if constexpr (CT) {
           if (own) {
             a.work[0][cell_p] = Fx[0];

@@ -62,13 +62,15 @@ __device__ __forceinline__ Edges mh_edges(const PortArgs& a, int i, int j, int k
   e.o[1] = recon<RECON_PLM>(load_prim(a, i, j - 1, k), m0, load_prim(a, i, j + 1, k));
   e.o[2] = recon<RECON_PLM>(load_prim(a, i, j, k - 1), m0, load_prim(a, i, j, k + 1));
   const F9 u0 = prim2cons(m0, a.P.gamma);
-  F9 acc = hancock_term<0, RECON_PLM>(m0, e.o[0], a.P.gamma);
-  acc = add9(acc, hancock_term<1, RECON_PLM>(m0, e.o[1], a.P.gamma));
-  acc = add9(acc, hancock_term<2, RECON_PLM>(m0, e.o[2], a.P.gamma));
+  P9 acc;
+  hancock_term<0, RECON_PLM, true>(acc, m0, e.o[0], a.P.gamma);
+  hancock_term<1, RECON_PLM, false>(acc, m0, e.o[1], a.P.gamma);
+  hancock_term<2, RECON_PLM, false>(acc, m0, e.o[2], a.P.gamma);
   const float h = 0.5f * a.dtdx;
   F9 uh;
 #pragma unroll
-  for (int v = 0; v < 9; ++v) uh[v] = u0[v] - h * acc[v];
+  for (int v = 0; v < 8; ++v) uh[v] = u0[v] - h * (acc[v].x - acc[v].y);
+  uh[8] = u0[8];
   e.mh = cons2prim(uh, a.P.gamma, a.P.smallr, a.P.pfl);
   return e;
 }
