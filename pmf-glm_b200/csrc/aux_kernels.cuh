@@ -2,6 +2,8 @@
 // the constrained-transport EMF / face / cell-B update, CT initialisation from a vector
 // potential, and the device-side CFL timestep for the batched driver.
 #pragma once
+#include <algorithm>
+
 #include "physics.cuh"
 
 namespace pmf {
@@ -46,59 +48,113 @@ static __global__ void __launch_bounds__(AUX_THREADS) wavespeed_kernel(const CPt
   if (threadIdx.x == 0) atomicMax(out_bits, __float_as_uint(m));
 }
 
-// max |div B| by BC-aware centred differences, in FP64 (diagnostics.jl:6-20)
+// Column launches of the div-B kernels: one thread per (x, y) column of a 32 x 8 tile marches `zc`
+// planes, so that a cell's index costs no division and the z neighbours stay in registers. zc is
+// the longest chunk (of at most 16 planes) that still gives every SM eight blocks.
+constexpr int COL_X = 32, COL_Y = AUX_THREADS / 32;
+inline dim3 col_grid(int nx, int ny, int nz, int sms, int* zc) {
+  const int tx = (nx + COL_X - 1) / COL_X, ty = (ny + COL_Y - 1) / COL_Y;
+  const long long chunks = std::max(1LL, std::min((long long)nz, 8LL * sms / ((long long)tx * ty)));
+  *zc = (int)std::min(16LL, (nz + chunks - 1) / chunks);
+  return dim3(tx, ty, (nz + *zc - 1) / *zc);
+}
+
+// max |div B| by BC-aware centred differences, in FP64 (diagnostics.jl:6-20).
+// In FP64 throughout, the conversions and adds of a cell cost several times its share of the
+// memory traffic, so a cell is evaluated in FP64 only where an FP32 evaluation leaves it a chance
+// to exceed the maximum so far (of its warp, and of the blocks that had finished when this one
+// began): the FP32 sum of the six terms is off by less than eight roundings of the sum of their
+// magnitudes. The result is the FP64 maximum, bit for bit. The maximum is kept without the factor
+// 1/(2 dx) until the end (rounding is monotonic, so the factor commutes with it).
 static __global__ void __launch_bounds__(AUX_THREADS) divb_kernel(const float* __restrict__ bx, const float* __restrict__ by,
-                                                           const float* __restrict__ bz, int nx, int ny, int nz,
+                                                           const float* __restrict__ bz, int nx, int ny, int nz, int zc,
                                                            int bcx, int bcy, int bcz, double inv2dx,
                                                            unsigned long long* out_bits) {
-  const int nc = nx * ny * nz;
+  const int ti = blockIdx.x * COL_X + (threadIdx.x & 31), tj = blockIdx.y * COL_Y + (threadIdx.x >> 5);
+  const bool in = ti < nx && tj < ny;
+  const int i = min(ti, nx - 1), j = min(tj, ny - 1);
+  float fxp, fxm, fyp, fym, fzm, fzp;
+  const unsigned row = (unsigned)j * nx, o = row + i;
+  const unsigned oxp = row + bc_index(i + 1, nx, bcx, &fxp), oxm = row + bc_index(i - 1, nx, bcx, &fxm);
+  const unsigned oyp = (unsigned)bc_index(j + 1, ny, bcy, &fyp) * nx + i;
+  const unsigned oym = (unsigned)bc_index(j - 1, ny, bcy, &fym) * nx + i;
+  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
+  const size_t nxy = (size_t)nx * ny;
+  const size_t top = bc_index(nz, nz, bcz, &fzp) * nxy;  // the plane above the last
   double m = 0.0;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-    const int i = c % nx, j = (c / nx) % ny, k = c / (nx * ny);
-    float fxp, fxm, fyp, fym, fzp, fzm;
-    const int ip = bc_index(i + 1, nx, bcx, &fxp), im = bc_index(i - 1, nx, bcx, &fxm);
-    const int jp = bc_index(j + 1, ny, bcy, &fyp), jm = bc_index(j - 1, ny, bcy, &fym);
-    const int kp = bc_index(k + 1, nz, bcz, &fzp), km = bc_index(k - 1, nz, bcz, &fzm);
-    auto L = [&](int a, int b, int d) { return (d * ny + b) * nx + a; };
-    const double db = ((double)bx[L(ip, j, k)] * fxp - (double)bx[L(im, j, k)] * fxm +
-                       (double)by[L(i, jp, k)] * fyp - (double)by[L(i, jm, k)] * fym +
-                       (double)bz[L(i, j, kp)] * fzp - (double)bz[L(i, j, km)] * fzm) * inv2dx;
-    m = fmax(m, fabs(db));
+  // a lower bound of the maximum (a millionth off, beyond the rounding of the division)
+  float lo = __double2float_rd(__longlong_as_double(*(volatile long long*)out_bits) / inv2dx * (1.0 - 1e-6));
+  const size_t below = bc_index(z0 - 1, nz, bcz, &fzm) * nxy;
+  float zm = bz[below + o] * fzm, z = bz[z0 * nxy + o];
+  for (int k = z0; k < z1; ++k) {
+    const float *xr = bx + k * nxy, *yr = by + k * nxy;
+    const bool last = k + 1 == nz;
+    const float zp = (bz + (last ? top : (k + 1) * nxy))[o] * (last ? fzp : 1.0f);
+    const float xp = xr[oxp] * fxp, xm = xr[oxm] * fxm, yp = yr[oyp] * fyp, ym = yr[oym] * fym;
+    const float d = (xp - xm) + (yp - ym) + (zp - zm);
+    const float mag = fabsf(xp) + fabsf(xm) + fabsf(yp) + fabsf(ym) + fabsf(zp) + fabsf(zm);
+    const bool maybe = in && fmaf(4.7683716e-7f, mag, fabsf(d)) >= lo;  // 2^-21 mag
+    if (maybe) {
+      const double db = (double)xp - (double)xm + (double)yp - (double)ym + (double)zp - (double)zm;
+      m = fmax(m, fabs(db));
+      lo = fmaxf(lo, __double2float_rd(m));
+    }
+    if (__any_sync(0xffffffffu, maybe)) lo = warp_max(lo);
+    zm = z;
+    z = zp;
   }
   m = block_reduce_max(m);
-  if (threadIdx.x == 0) atomicMax(out_bits, (unsigned long long)__double_as_longlong(m));
+  if (threadIdx.x == 0) atomicMax(out_bits, (unsigned long long)__double_as_longlong(m * inv2dx));
 }
 
 // max face divergence of a CT face field, FP64 (ct.jl:176-185)
 static __global__ void __launch_bounds__(AUX_THREADS) divb_face_kernel(const float* __restrict__ bxf,
                                                                 const float* __restrict__ byf,
                                                                 const float* __restrict__ bzf, int nx, int ny,
-                                                                int nz, double invdx,
+                                                                int nz, int zc, double invdx,
                                                                 unsigned long long* out_bits) {
-  const int nc = nx * ny * nz;
+  const int i = blockIdx.x * COL_X + (threadIdx.x & 31), j = blockIdx.y * COL_Y + (threadIdx.x >> 5);
   double m = 0.0;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-    const int i = c % nx, j = (c / nx) % ny, k = c / (nx * ny);
-    const int nxy = nx * ny;
-    const double d = (((double)bxf[k * nxy + j * nx + wrap_inc(i, nx)] - bxf[c]) +
-                      ((double)byf[k * nxy + wrap_inc(j, ny) * nx + i] - byf[c]) +
-                      ((double)bzf[wrap_inc(k, nz) * nxy + j * nx + i] - bzf[c])) * invdx;
-    m = fmax(m, fabs(d));
+  if (i < nx && j < ny) {
+    const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
+    const size_t nxy = (size_t)nx * ny, o = (size_t)j * nx + i;
+    const size_t oip = (size_t)j * nx + wrap_inc(i, nx), ojp = (size_t)wrap_inc(j, ny) * nx + i;
+    float z = bzf[z0 * nxy + o];
+    for (int k = z0; k < z1; ++k) {
+      const size_t b = k * nxy;
+      const float zp = bzf[wrap_inc(k, nz) * nxy + o];
+      const double d = (((double)bxf[b + oip] - bxf[b + o]) + ((double)byf[b + ojp] - byf[b + o]) + ((double)zp - z)) * invdx;
+      m = fmax(m, fabs(d));
+      z = zp;
+    }
   }
   m = block_reduce_max(m);
   if (threadIdx.x == 0) atomicMax(out_bits, (unsigned long long)__double_as_longlong(m));
 }
 
 // Deterministic FP64 field sums: per-block partials (fixed order), then one block folds them.
+// V4: four cells a load (16-byte aligned fields of a multiple of four cells); the kernel is bound
+// by HBM, and eight scalar loads a thread keep too little in flight.
+template <bool V4>
 static __global__ void __launch_bounds__(AUX_THREADS) totals_partial_kernel(const CPtr9 U, int nc,
                                                                      double* partial) {
   __shared__ double red[AUX_THREADS / 32][8];
   double s[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) s[q] = 0.0;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
+  if constexpr (V4) {
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc / 4; c += gridDim.x * blockDim.x) {
+      float4 v[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) s[q] += (double)__ldg(U.p[q] + c);
+      for (int q = 0; q < 8; ++q) v[q] = __ldg(reinterpret_cast<const float4*>(U.p[q]) + c);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) s[q] += ((double)v[q].x + (double)v[q].y) + ((double)v[q].z + (double)v[q].w);
+    }
+  } else {
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) s[q] += (double)__ldg(U.p[q] + c);
+    }
   }
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
@@ -114,12 +170,19 @@ static __global__ void __launch_bounds__(AUX_THREADS) totals_partial_kernel(cons
     partial[blockIdx.x * 8 + threadIdx.x] = t;
   }
 }
-static __global__ void totals_final_kernel(const double* partial, int nblocks, double scale, double* out) {
-  if (threadIdx.x < 8) {
-    double t = 0.0;
-    for (int b = 0; b < nblocks; ++b) t += partial[b * 8 + threadIdx.x];
-    out[threadIdx.x] = t * scale;
+// AUX_THREADS threads: thread t folds the partials of sum t % 8 of the blocks t / 8, t / 8 + 32, ...
+// (one thread per sum took a serial chain of up to 1024 FP64 adds)
+static __global__ void __launch_bounds__(AUX_THREADS) totals_final_kernel(const double* partial, int nblocks, double scale,
+                                                                   double* out) {
+  __shared__ double red[AUX_THREADS];
+  double t = 0.0;
+  for (int b = threadIdx.x >> 3; b < nblocks; b += AUX_THREADS / 8) t += partial[b * 8 + (threadIdx.x & 7)];
+  red[threadIdx.x] = t;
+  for (int n = AUX_THREADS / 2; n >= 8; n >>= 1) {
+    __syncthreads();
+    if ((int)threadIdx.x < n) red[threadIdx.x] += red[threadIdx.x + n];
   }
+  if (threadIdx.x < 8) out[threadIdx.x] = red[threadIdx.x] * scale;
 }
 
 // ---- constrained transport (ct.jl:57-143) ------------------------------------------------

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -621,9 +622,10 @@ int pmfmhd_max_divb(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const U[9]
   if (!nonnull(U, 9)) return PMFMHD_EINVAL;
   cudaStream_t s = as_stream(stream);
   PMF_CK(cudaMemsetAsync(c->d_u64, 0, sizeof(unsigned long long), s));
-  divb_kernel<<<aux_blocks(c, ncells(g)), AUX_THREADS, 0, s>>>(U[5], U[6], U[7], g->nx, g->ny, g->nz, g->bc[0],
-                                                                g->bc[1], g->bc[2], 1.0 / (2.0 * (double)g->dx),
-                                                                c->d_u64);
+  int zc;
+  const dim3 tiles = col_grid(g->nx, g->ny, g->nz, c->sms, &zc);
+  divb_kernel<<<tiles, AUX_THREADS, 0, s>>>(U[5], U[6], U[7], g->nx, g->ny, g->nz, zc, g->bc[0], g->bc[1], g->bc[2],
+                                            1.0 / (2.0 * (double)g->dx), c->d_u64);
   PMF_CK(cudaGetLastError());
   PMF_CK(cudaMemcpyAsync(c->h_pin, c->d_u64, 8, cudaMemcpyDeviceToHost, s));
   PMF_CK(cudaStreamSynchronize(s));
@@ -638,8 +640,10 @@ int pmfmhd_max_divb_face(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* ct, d
   cudaStream_t s = as_stream(stream);
   const long long nc = ncells(g);
   PMF_CK(cudaMemsetAsync(c->d_u64, 0, sizeof(unsigned long long), s));
-  divb_face_kernel<<<aux_blocks(c, nc), AUX_THREADS, 0, s>>>(ct, ct + nc, ct + 2 * nc, g->nx, g->ny, g->nz,
-                                                              1.0 / (double)g->dx, c->d_u64);
+  int zc;
+  const dim3 tiles = col_grid(g->nx, g->ny, g->nz, c->sms, &zc);
+  divb_face_kernel<<<tiles, AUX_THREADS, 0, s>>>(ct, ct + nc, ct + 2 * nc, g->nx, g->ny, g->nz, zc,
+                                                 1.0 / (double)g->dx, c->d_u64);
   PMF_CK(cudaGetLastError());
   PMF_CK(cudaMemcpyAsync(c->h_pin, c->d_u64, 8, cudaMemcpyDeviceToHost, s));
   PMF_CK(cudaStreamSynchronize(s));
@@ -656,10 +660,14 @@ int pmfmhd_conserved_totals(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* co
   cudaStream_t s = as_stream(stream);
   CPtr9 u;
   for (int f = 0; f < 9; ++f) u.p[f] = U[f];
-  const int nb = std::min(aux_blocks(c, ncells(g)), kTotBlocksMax);
-  totals_partial_kernel<<<nb, AUX_THREADS, 0, s>>>(u, (int)ncells(g), c->d_partial);
+  const long long nc = ncells(g);
+  bool v4 = nc % 4 == 0;
+  for (int f = 0; f < 8; ++f) v4 = v4 && reinterpret_cast<uintptr_t>(U[f]) % 16 == 0;
+  const int nb = std::min(aux_blocks(c, v4 ? nc / 4 : nc), kTotBlocksMax);
+  if (v4) totals_partial_kernel<true><<<nb, AUX_THREADS, 0, s>>>(u, (int)nc, c->d_partial);
+  else totals_partial_kernel<false><<<nb, AUX_THREADS, 0, s>>>(u, (int)nc, c->d_partial);
   const float dV = g->dx * g->dx * g->dx;  // s.dx^3 in T (diagnostics.jl:45)
-  totals_final_kernel<<<1, 32, 0, s>>>(c->d_partial, nb, (double)dV, c->d_tot);
+  totals_final_kernel<<<1, AUX_THREADS, 0, s>>>(c->d_partial, nb, (double)dV, c->d_tot);
   PMF_CK(cudaGetLastError());
   PMF_CK(cudaMemcpyAsync(c->h_pin, c->d_tot, 64, cudaMemcpyDeviceToHost, s));
   PMF_CK(cudaStreamSynchronize(s));
