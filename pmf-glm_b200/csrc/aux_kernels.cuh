@@ -34,7 +34,8 @@ template <class T> __device__ __forceinline__ T block_reduce_max(T v) {
   return v;
 }
 
-// max over cells of max_d(|v_d| + c_f,d)  (timestep.jl:4-14), one atomic per block
+// max over cells of max_d(|v_d| + c_f,d)  (timestep.jl:4-14): block b's maximum in out_bits[b + 1],
+// the blocks less one in out_bits[0]
 static __global__ void __launch_bounds__(AUX_THREADS) wavespeed_kernel(const CPtr9 U, int nc, Phys P,
                                                                 unsigned int* out_bits) {
   float m = 0.0f;
@@ -45,7 +46,10 @@ static __global__ void __launch_bounds__(AUX_THREADS) wavespeed_kernel(const CPt
     m = fmaxf(m, cell_wavespeed(u, P));
   }
   m = block_reduce_max(m);
-  if (threadIdx.x == 0) atomicMax(out_bits, __float_as_uint(m));
+  if (threadIdx.x == 0) {
+    out_bits[blockIdx.x + 1] = __float_as_uint(m);
+    if (blockIdx.x == 0) out_bits[0] = gridDim.x - 1;
+  }
 }
 
 // Column launches of the div-B kernels: one thread per (x, y) column of a 32 x 8 tile marches `zc`
@@ -204,15 +208,23 @@ enum { CT_BXF = 0, CT_BYF, CT_BZF, CT_MFX, CT_MFY, CT_MFZ, CT_FXBY, CT_FXBZ, CT_
        CT_ECX, CT_ECY, CT_ECZ, CT_EX, CT_EY, CT_EZ, CT_RBX, CT_RBY, CT_RBZ, CT_NSLOT };
 
 // ---- CT companion kernels: column forms -------------------------------------------------
-// One thread per (x, y) column of a 32 x 8 tile marches a chunk of CTC_Z planes in z: the
+// One thread per (x, y) column of a 32 x 8 tile marches a chunk of zc planes in z: the
 // cell index needs no division, every slot has its own restrict pointer (so the compiler
 // may overlap one plane's loads with the last plane's stores), and the values of plane k
 // that plane k+1 reads again as its lower neighbour stay in registers (25 loads per cell
 // for the EMFs, of the 36 values its stencil touches). Per cell: the Gardiner & Stone EMFs (ct.jl:71-93), the face
 // update (ct.jl:96-129) and the face-average cell B (ct.jl:132-143).
-constexpr int CTC_X = 32, CTC_Y = AUX_THREADS / 32, CTC_Z = 16;
+constexpr int CTC_X = 32, CTC_Y = AUX_THREADS / 32, CTC_Z = 16;  // CTC_Z: the longest chunk
 inline dim3 ctc_grid(int nx, int ny, int nz) {
   return dim3((nx + CTC_X - 1) / CTC_X, (ny + CTC_Y - 1) / CTC_Y, (nz + CTC_Z - 1) / CTC_Z);
+}
+// One box alone: chunks short enough that a small box still gives every SM eight blocks (the
+// planes of a chunk are serial; at 16 planes the three kernels of a 48^3 step took 27 us).
+inline dim3 ctc_grid(int nx, int ny, int nz, int sms, int* zc) {
+  const dim3 t = ctc_grid(nx, ny, nz);
+  const long long chunks = std::max(1LL, std::min((long long)nz, 8LL * sms / ((long long)t.x * t.y)));
+  *zc = (int)std::min((long long)CTC_Z, (nz + chunks - 1) / chunks);
+  return dim3(t.x, t.y, (nz + *zc - 1) / *zc);
 }
 
 // The column bodies: tile (tx, ty), z chunk tz; thread t of AUX_THREADS owns column
@@ -226,10 +238,10 @@ __device__ __forceinline__ void ct_emf_col(
     const float* __restrict__ FYBZ, const float* __restrict__ FZBX, const float* __restrict__ FZBY,
     const float* __restrict__ ECX, const float* __restrict__ ECY, const float* __restrict__ ECZ,
     float* __restrict__ EX, float* __restrict__ EY, float* __restrict__ EZ, int nx, int ny, int nz, int tx, int ty,
-    int tz) {
+    int tz, int zc) {
   const int i = tx * CTC_X + (threadIdx.x & 31), j = ty * CTC_Y + (threadIdx.x >> 5);
   if (i >= nx || j >= ny) return;
-  const int z0 = tz * CTC_Z, z1 = min(z0 + CTC_Z, nz);
+  const int z0 = tz * zc, z1 = min(z0 + zc, nz);
   const size_t nxy = (size_t)nx * ny;
   const int im = wrap_dec(i, nx), jm = wrap_dec(j, ny);
   const size_t o = (size_t)j * nx + i, oim = (size_t)j * nx + im, ojm = (size_t)jm * nx + i,
@@ -261,10 +273,10 @@ __device__ __forceinline__ void ct_face_col(const float* __restrict__ ex, const 
                                             const float* __restrict__ ez, float* __restrict__ bxf,
                                             float* __restrict__ byf, float* __restrict__ bzf, float* __restrict__ rbx,
                                             float* __restrict__ rby, float* __restrict__ rbz, int nx, int ny, int nz,
-                                            float dtdx, int tx, int ty, int tz) {
+                                            float dtdx, int tx, int ty, int tz, int zc) {
   const int i = tx * CTC_X + (threadIdx.x & 31), j = ty * CTC_Y + (threadIdx.x >> 5);
   if (i >= nx || j >= ny) return;
-  const int z0 = tz * CTC_Z, z1 = min(z0 + CTC_Z, nz);
+  const int z0 = tz * zc, z1 = min(z0 + zc, nz);
   const size_t nxy = (size_t)nx * ny;
   const size_t o = (size_t)j * nx + i, oip = (size_t)j * nx + wrap_inc(i, nx), ojp = (size_t)wrap_inc(j, ny) * nx + i;
   // plane k values that plane k-1 read as its upper neighbour
@@ -300,11 +312,12 @@ __device__ __forceinline__ void ct_face_col(const float* __restrict__ ex, const 
 // state (0 without want_speed). Every thread returns: the caller reduces over the block.
 __device__ __forceinline__ float ct_bcc_col(const float* __restrict__ bxf, const float* __restrict__ byf,
                                             const float* __restrict__ bzf, const MPtr9& Un, int nx, int ny, int nz,
-                                            const Phys& P, bool want_speed, int tx, int ty, int tz) {
+                                            const Phys& P, bool want_speed, int tx, int ty, int tz,
+                                            int zc) {
   const int i = tx * CTC_X + (threadIdx.x & 31), j = ty * CTC_Y + (threadIdx.x >> 5);
   float m = 0.0f;
   if (i >= nx || j >= ny) return m;
-  const int z0 = tz * CTC_Z, z1 = min(z0 + CTC_Z, nz);
+  const int z0 = tz * zc, z1 = min(z0 + zc, nz);
   const size_t nxy = (size_t)nx * ny;
   const size_t o = (size_t)j * nx + i, oip = (size_t)j * nx + wrap_inc(i, nx), ojp = (size_t)wrap_inc(j, ny) * nx + i;
   float bz_c = bzf[(size_t)z0 * nxy + o];
@@ -331,23 +344,26 @@ static __global__ void __launch_bounds__(AUX_THREADS) ct_emf_col_kernel(
     const float* __restrict__ FXBY, const float* __restrict__ FXBZ, const float* __restrict__ FYBX,
     const float* __restrict__ FYBZ, const float* __restrict__ FZBX, const float* __restrict__ FZBY,
     const float* __restrict__ ECX, const float* __restrict__ ECY, const float* __restrict__ ECZ,
-    float* __restrict__ EX, float* __restrict__ EY, float* __restrict__ EZ, int nx, int ny, int nz) {
+    float* __restrict__ EX, float* __restrict__ EY, float* __restrict__ EZ, int nx, int ny, int nz,
+    int zc, unsigned int* __restrict__ smax) {
+  // the signal-speed cell that ct_bcc_col_kernel raises two launches later: one entry, 0
+  if (threadIdx.x < 2 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) smax[threadIdx.x] = 0u;
   ct_emf_col(MFX, MFY, MFZ, FXBY, FXBZ, FYBX, FYBZ, FZBX, FZBY, ECX, ECY, ECZ, EX, EY, EZ, nx, ny, nz, blockIdx.x,
-             blockIdx.y, blockIdx.z);
+             blockIdx.y, blockIdx.z, zc);
 }
 
 template <bool COMP>
 static __global__ void __launch_bounds__(AUX_THREADS) ct_face_col_kernel(
     const float* __restrict__ ex, const float* __restrict__ ey, const float* __restrict__ ez,
     float* __restrict__ bxf, float* __restrict__ byf, float* __restrict__ bzf, float* __restrict__ rbx,
-    float* __restrict__ rby, float* __restrict__ rbz, int nx, int ny, int nz, float dtdx) {
-  ct_face_col<COMP>(ex, ey, ez, bxf, byf, bzf, rbx, rby, rbz, nx, ny, nz, dtdx, blockIdx.x, blockIdx.y, blockIdx.z);
+    float* __restrict__ rby, float* __restrict__ rbz, int nx, int ny, int nz, int zc, float dtdx) {
+  ct_face_col<COMP>(ex, ey, ez, bxf, byf, bzf, rbx, rby, rbz, nx, ny, nz, dtdx, blockIdx.x, blockIdx.y, blockIdx.z, zc);
 }
 
 static __global__ void __launch_bounds__(AUX_THREADS) ct_bcc_col_kernel(
     const float* __restrict__ bxf, const float* __restrict__ byf, const float* __restrict__ bzf, const MPtr9 Un,
-    int nx, int ny, int nz, Phys P, unsigned int* smax_bits) {
-  float m = ct_bcc_col(bxf, byf, bzf, Un, nx, ny, nz, P, smax_bits != nullptr, blockIdx.x, blockIdx.y, blockIdx.z);
+    int nx, int ny, int nz, int zc, Phys P, unsigned int* smax_bits) {
+  float m = ct_bcc_col(bxf, byf, bzf, Un, nx, ny, nz, P, smax_bits != nullptr, blockIdx.x, blockIdx.y, blockIdx.z, zc);
   if (smax_bits != nullptr) {
     m = block_reduce_max(m);
     if (threadIdx.x == 0) atomicMax(smax_bits, __float_as_uint(m));

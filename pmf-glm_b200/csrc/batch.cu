@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(AUX_THREADS) batch_ct_emf_kernel(const CtView*
   ct_emf_col(ct_slot(b, CT_MFX), ct_slot(b, CT_MFY), ct_slot(b, CT_MFZ), ct_slot(b, CT_FXBY), ct_slot(b, CT_FXBZ),
              ct_slot(b, CT_FYBX), ct_slot(b, CT_FYBZ), ct_slot(b, CT_FZBX), ct_slot(b, CT_FZBY), ct_slot(b, CT_ECX),
              ct_slot(b, CT_ECY), ct_slot(b, CT_ECZ), ct_slot(b, CT_EX), ct_slot(b, CT_EY), ct_slot(b, CT_EZ), b.nx,
-             b.ny, b.nz, tx, ty, tz);
+             b.ny, b.nz, tx, ty, tz, CTC_Z);
 }
 
 __global__ void __launch_bounds__(AUX_THREADS) batch_ct_face_kernel(const CtView* __restrict__ v, int n) {
@@ -88,11 +88,11 @@ __global__ void __launch_bounds__(AUX_THREADS) batch_ct_face_kernel(const CtView
   if (b.comp_faces)
     ct_face_col<true>(ct_slot(b, CT_EX), ct_slot(b, CT_EY), ct_slot(b, CT_EZ), ct_slot(b, CT_BXF), ct_slot(b, CT_BYF),
                       ct_slot(b, CT_BZF), ct_slot(b, CT_RBX), ct_slot(b, CT_RBY), ct_slot(b, CT_RBZ), b.nx, b.ny,
-                      b.nz, dtdx, tx, ty, tz);
+                      b.nz, dtdx, tx, ty, tz, CTC_Z);
   else
     ct_face_col<false>(ct_slot(b, CT_EX), ct_slot(b, CT_EY), ct_slot(b, CT_EZ), ct_slot(b, CT_BXF),
                        ct_slot(b, CT_BYF), ct_slot(b, CT_BZF), ct_slot(b, CT_RBX), ct_slot(b, CT_RBY),
-                       ct_slot(b, CT_RBZ), b.nx, b.ny, b.nz, dtdx, tx, ty, tz);
+                       ct_slot(b, CT_RBZ), b.nx, b.ny, b.nz, dtdx, tx, ty, tz, CTC_Z);
 }
 
 __global__ void __launch_bounds__(AUX_THREADS) batch_ct_bcc_kernel(const CtView* __restrict__ v, int n) {
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(AUX_THREADS) batch_ct_bcc_kernel(const CtView*
   int tx, ty, tz;
   col_tile(b, blockIdx.x, tx, ty, tz);
   float m = ct_bcc_col(ct_slot(b, CT_BXF), ct_slot(b, CT_BYF), ct_slot(b, CT_BZF), b.Un, b.nx, b.ny, b.nz, b.P, true,
-                       tx, ty, tz);
+                       tx, ty, tz, CTC_Z);
   m = block_reduce_max(m);
   if (threadIdx.x == 0) atomicMax(b.smax_bits, __float_as_uint(m));
 }
@@ -250,7 +250,7 @@ int pmfmhd_batch_create(pmfmhd_ctx* c, const pmfmhd_box* boxes, int nbox, pmfmhd
       const long long nc = ncells(&x.grid);
       if (nc > family_cells[fam]) {
         family_cells[fam] = nc;
-        family_ty[fam] = tune_for(c, &x.grid, ct, comp).ty;
+        family_ty[fam] = batch_tune(c, &x.grid, ct, comp).ty;
       }
     }
   }
@@ -259,7 +259,7 @@ int pmfmhd_batch_create(pmfmhd_ctx* c, const pmfmhd_box* boxes, int nbox, pmfmhd
   for (int i = 0; i < nbox; ++i) {
     const pmfmhd_box& x = boxes[i];
     const bool ct = x.mhd_solver == 1, comp = x.resid[0] != nullptr;
-    Tune t = tune_for(c, &x.grid, ct, comp);
+    Tune t = batch_tune(c, &x.grid, ct, comp);
     t.ty = family_ty[std::make_tuple((int)ct, (int)comp, x.grid.recon, x.grid.riemann)];
     auto key = std::make_tuple((int)ct, (int)comp, x.grid.recon, x.grid.riemann, t.ty);
     if (!gidx.count(key)) {

@@ -23,6 +23,8 @@ using namespace pmf::host;
 
 namespace {
 constexpr int kTotBlocksMax = 1024;
+// Entries of the signal-speed array: a count and one maximum per CTA (at most eight per SM).
+constexpr int kSmaxMax = 2048;
 }  // namespace
 
 namespace pmf {
@@ -85,20 +87,77 @@ int aux_blocks(const pmfmhd_ctx* c, long long nc) {
   return (int)(b < cap ? (b < 1 ? 1 : b) : cap);
 }
 
-// Tile height and the minimum number of planes per CTA (the launch gives every CTA an
-// equal share of the (column, plane) space, but never less than `tz` planes).
-Tune default_tune(const pmfmhd_ctx*, const pmfmhd_grid* g) {
-  Tune t;
-  t.ty = g->ny >= 8 ? 8 : 5;
-  t.tz = 16;
-  return t;
+// How a launch divides its `cols` column tiles of `nz` planes over at most `slots` resident CTAs
+// of at least `tz` planes each: equal parts of every column (no CTA has a second column segment),
+// or an even share of the concatenated planes whatever columns it crosses (more CTAs busy where
+// the columns do not divide the slots well). A segment costs about three planes beyond its own:
+// its first three planes are staged and its end planes predicted before it owns anything. The
+// cheaper of the two by the planes of the longest CTA.
+struct Split {
+  int zparts;         // StepArgs::zparts
+  int blocks;
+  long long longest;  // planes of the longest CTA, its segments' overhead included
+};
+Split split_work(long long cols, int nz, long long slots, int tz) {
+  constexpr long long kSegment = 3;
+  tz = std::max(1, std::min(tz, nz));
+  const long long Q = cols * nz;
+  Split s;
+  s.zparts = 0;
+  s.blocks = (int)std::min(slots, std::max<long long>(1, Q / tz));
+  const long long share = (Q + s.blocks - 1) / s.blocks;
+  s.longest = share + (share / nz + 2) * kSegment;  // a share crosses into at least a second column
+  if (cols <= slots) {
+    const long long parts = std::min<long long>(slots / cols, std::max(1, nz / tz));
+    const long long longest = (nz + parts - 1) / parts + kSegment;
+    if (longest <= s.longest) s = Split{(int)parts, (int)(cols * parts), longest};
+  }
+  return s;
 }
 
-Tune tune_for(pmfmhd_ctx* c, const pmfmhd_grid* g, bool ct, bool comp) {
+// Tile height of an untuned grid: the height whose longest CTA takes least, its planes times the
+// relative time of one plane of a full GPU. Measured at 256^3: 3.4, 3.85 us a plane at 8 and 9
+// rows for GLM, 3.5, 4.15 for CT, 6.2, 6.8, 8.9 at 8, 9 and 13 for the radiation-coupled step
+// (which waits on its loads of the correction arrays, so that its 16 warps at 13 rows pay; the
+// others are slower at 13 rows for every size). A grid under 8 rows takes the 5-row tile.
+Tune default_tune(const pmfmhd_ctx* c, const pmfmhd_grid* g, bool ct, int src) {
+  if (g->ny < 8) return Tune{5, 1};
+  struct Cost {
+    int ty;
+    double glm, ct, rad;
+  };
+  constexpr Cost kCost[] = {{8, 1.0, 1.0, 1.0}, {9, 1.13, 1.18, 1.09}, {13, 1e9, 1e9, 1.43}};
+  Tune best{8, 1};
+  double least = 1e300;
+  for (const Cost& k : kCost) {
+    const long long cols = (long long)((g->nx + TILE_X - 1) / TILE_X) * ((g->ny + k.ty - 1) / k.ty);
+    const double cost = (double)split_work(cols, g->nz, c->sms, 1).longest * (src == SRC_RAD ? k.rad : ct ? k.ct : k.glm);
+    if (cost < least) {
+      least = cost;
+      best.ty = k.ty;
+    }
+  }
+  return best;
+}
+
+bool tuned(pmfmhd_ctx* c, const pmfmhd_grid* g, bool ct, bool comp, Tune* t) {
   std::lock_guard<std::mutex> lk(c->mu);
   auto it = c->tune.find(TuneKey{g->nx, g->ny, g->nz, ct, comp, g->recon, g->riemann});
-  if (it != c->tune.end()) return it->second;
-  return default_tune(c, g);
+  if (it == c->tune.end()) return false;
+  *t = it->second;
+  return true;
+}
+
+Tune tune_for(pmfmhd_ctx* c, const pmfmhd_grid* g, bool ct, bool comp, int src) {
+  Tune t;
+  return tuned(c, g, ct, comp, &t) ? t : default_tune(c, g, ct, src);
+}
+
+// In a batch the boxes share the persistent CTAs and the split of one box does not matter: 8 rows
+// (the fewest halo rows that keep the update's loads a pass ahead) unless the box was tuned.
+Tune batch_tune(pmfmhd_ctx* c, const pmfmhd_grid* g, bool ct, bool comp) {
+  Tune t;
+  return tuned(c, g, ct, comp, &t) ? t : Tune{g->ny >= 8 ? 8 : 5, 1};
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link to libcuda).
@@ -174,18 +233,17 @@ int launch_step(pmfmhd_ctx* c, const pmfmhd_grid* g, StepArgs& a, Tune t, bool c
   a.P = phys_of(g);
   a.status = c->d_status;
   a.tma_stall_polls = c->tma_stall_polls;
-  // Interior planes come in by TMA for the plain and compensated GLM step; the CT and
-  // source-coupled instantiations are compiled without the TMA path and stage every plane by
-  // per-element cp.async.
-  a.use_tma = (!ct && src == SRC_NONE && field_maps(c, g, a.U, t.ty, a.tmap)) ? 1 : 0;
+  // Interior planes come in by TMA for the plain GLM step; the other instantiations are compiled
+  // without the TMA path and stage every plane by per-element cp.async.
+  a.use_tma = (!ct && !comp && src == SRC_NONE && field_maps(c, g, a.U, t.ty, a.tmap)) ? 1 : 0;
   if (a.zhi <= a.zlo) {  // the whole box unless the caller set a plane range
     a.zlo = 0;
     a.zhi = g->nz;
   }
-  const long long Q = (long long)a.ntx * a.nty * (a.zhi - a.zlo);
-  const long long slots = (long long)c->sms * occ;
-  const long long by_work = std::max<long long>(1, (Q + t.tz - 1) / std::max(1, t.tz));
-  const long long blocks = std::min(slots, by_work);
+  const Split sp =
+      split_work((long long)a.ntx * a.nty, a.zhi - a.zlo, std::min((long long)c->sms * occ, kSmaxMax - 1LL), t.tz);
+  a.zparts = sp.zparts;
+  const int blocks = sp.blocks;
   void* args[] = {(void*)&a};
   PMF_CK(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)blocks), dim3(k.threads), args, k.smem_bytes, s));
   return PMFMHD_OK;
@@ -199,6 +257,7 @@ void fill_glm_args(StepArgs& a, const float* const U[9], float* const Un[9], flo
     for (int i = 0; i < 7; ++i) a.resid[i] = resid[i];
   a.dtdx = dtdx; a.ch = ch; a.decay = decay;
   a.smax_bits = smax_bits;
+  a.smax_part = 1;
   a.dscal = nullptr;
 }
 
@@ -251,8 +310,8 @@ int enqueue_glm(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const U[9], fl
   const float dtdx = dt / g->dx;  // T(dt)/s.dx (integrator_ref.jl:211)
   fill_glm_args(a, U, Un, resid, comp, dtdx, ch, decay, c->d_smax);
   apply_sources(a, st);
-  PMF_CK(cudaMemsetAsync(c->d_smax, 0, sizeof(unsigned int), s));
-  return launch_step(c, g, a, tune_for(c, g, false, comp), false, comp, s, st ? st->src : SRC_NONE);
+  const int src = st ? st->src : SRC_NONE;
+  return launch_step(c, g, a, tune_for(c, g, false, comp, src), false, comp, s, src);
 }
 
 int enqueue_ct(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const U[9], float* const Un[9], float* ct, float dt,
@@ -264,39 +323,40 @@ int enqueue_ct(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const U[9], flo
   apply_sources(a, st);
   for (int d = 0; d < 3; ++d) a.face[d] = ct + (size_t)(CT_BXF + d) * nc;
   for (int k = 0; k < CT_NWORK; ++k) a.work[k] = ct + (size_t)(CT_MFX + k) * nc;
-  int rc = launch_step(c, g, a, tune_for(c, g, true, comp), true, comp, s, st ? st->src : SRC_NONE);
+  const int src = st ? st->src : SRC_NONE;
+  int rc = launch_step(c, g, a, tune_for(c, g, true, comp, src), true, comp, s, src);
   if (rc != PMFMHD_OK) return rc;
   auto sl = [&](int k) { return ct + (size_t)k * nc; };
-  const dim3 cg = ctc_grid(g->nx, g->ny, g->nz);
+  int zc;
+  const dim3 cg = ctc_grid(g->nx, g->ny, g->nz, c->sms, &zc);
   ct_emf_col_kernel<<<cg, AUX_THREADS, 0, s>>>(sl(CT_MFX), sl(CT_MFY), sl(CT_MFZ), sl(CT_FXBY), sl(CT_FXBZ),
                                                sl(CT_FYBX), sl(CT_FYBZ), sl(CT_FZBX), sl(CT_FZBY), sl(CT_ECX),
                                                sl(CT_ECY), sl(CT_ECZ), sl(CT_EX), sl(CT_EY), sl(CT_EZ), g->nx,
-                                               g->ny, g->nz);
+                                               g->ny, g->nz, zc, c->d_smax);
   if (comp_faces)
     ct_face_col_kernel<true><<<cg, AUX_THREADS, 0, s>>>(sl(CT_EX), sl(CT_EY), sl(CT_EZ), sl(CT_BXF), sl(CT_BYF),
-                                                        sl(CT_BZF), sl(CT_RBX), sl(CT_RBY), sl(CT_RBZ), g->nx,
-                                                        g->ny, g->nz, dtdx);
+                                                        sl(CT_BZF), sl(CT_RBX), sl(CT_RBY), sl(CT_RBZ), g->nx, g->ny, g->nz,
+                                                        zc, dtdx);
   else
     ct_face_col_kernel<false><<<cg, AUX_THREADS, 0, s>>>(sl(CT_EX), sl(CT_EY), sl(CT_EZ), sl(CT_BXF), sl(CT_BYF),
-                                                         sl(CT_BZF), sl(CT_RBX), sl(CT_RBY), sl(CT_RBZ), g->nx,
-                                                         g->ny, g->nz, dtdx);
-  PMF_CK(cudaMemsetAsync(c->d_smax, 0, sizeof(unsigned int), s));
+                                                         sl(CT_BZF), sl(CT_RBX), sl(CT_RBY), sl(CT_RBZ), g->nx, g->ny, g->nz,
+                                                        zc, dtdx);
   MPtr9 un;
   for (int f = 0; f < 9; ++f) un.p[f] = Un[f];
   ct_bcc_col_kernel<<<cg, AUX_THREADS, 0, s>>>(sl(CT_BXF), sl(CT_BYF), sl(CT_BZF), un, g->nx, g->ny, g->nz,
-                                               phys_of(g), c->d_smax);
+                                               zc, phys_of(g), c->d_smax + 1);
   PMF_CK(cudaGetLastError());
   return PMFMHD_OK;
 }
 
+// The maximum of the signal-speed array (entry 0: the maxima that follow, less one).
 int read_smax(pmfmhd_ctx* c, float* out, cudaStream_t s) {
-  PMF_CK(cudaMemcpyAsync(c->h_pin, c->d_smax, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+  PMF_CK(cudaMemcpyAsync(c->h_pin, c->d_smax, kSmaxMax * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
   PMF_CK(cudaStreamSynchronize(s));
-  unsigned int bits;
-  std::memcpy(&bits, c->h_pin, sizeof(bits));
-  float v;
-  std::memcpy(&v, &bits, sizeof(v));
-  *out = v;
+  const unsigned int* bits = reinterpret_cast<const unsigned int*>(c->h_pin);
+  const unsigned int n = std::min(bits[0] + 1, (unsigned int)kSmaxMax - 1);
+  const unsigned int m = *std::max_element(bits + 1, bits + 1 + n);  // non-negative floats order as their bits
+  std::memcpy(out, &m, sizeof(m));
   return PMFMHD_OK;
 }
 
@@ -330,16 +390,16 @@ int pmfmhd_create(int device, pmfmhd_ctx** out) {
   pmfmhd_ctx* c = new pmfmhd_ctx();
   c->device = device;
   if (cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) c->sms = 148;
-  if (cudaMalloc(&c->d_smax, 256) != cudaSuccess || cudaMalloc(&c->d_u64, 256) != cudaSuccess ||
+  if (cudaMalloc(&c->d_smax, kSmaxMax * sizeof(unsigned int)) != cudaSuccess || cudaMalloc(&c->d_u64, 256) != cudaSuccess ||
       cudaMalloc(&c->d_partial, sizeof(double) * 8 * kTotBlocksMax) != cudaSuccess ||
-      cudaMalloc(&c->d_tot, sizeof(double) * 8) != cudaSuccess || cudaMallocHost(&c->h_pin, 256) != cudaSuccess ||
+      cudaMalloc(&c->d_tot, sizeof(double) * 8) != cudaSuccess || cudaMallocHost(&c->h_pin, kSmaxMax * sizeof(unsigned int)) != cudaSuccess ||
       cudaMalloc(&c->d_status, sizeof(unsigned int)) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->cap, cudaStreamNonBlocking) != cudaSuccess) {
     last_cuda_error() = cudaGetErrorString(cudaGetLastError());
     pmfmhd_destroy(c);
     return PMFMHD_ENOMEM;
   }
-  PMF_CK(cudaMemset(c->d_smax, 0, 256));
+  PMF_CK(cudaMemset(c->d_smax, 0, kSmaxMax * sizeof(unsigned int)));
   PMF_CK(cudaMemset(c->d_status, 0, sizeof(unsigned int)));
   *out = c;
   return PMFMHD_OK;
@@ -458,11 +518,12 @@ int pmfmhd_step_glm_host(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const
   // compute chunk k once chunks k-1, k, k+1 (periodic) are resident; copy it out as soon as done
   const float dtdx = dt / g->dx;
   const Tune t = tune_for(c, g, false, false);
-  PMF_CK(cudaMemsetAsync(c->d_smax, 0, sizeof(unsigned int), scomp));
+  PMF_CK(cudaMemsetAsync(c->d_smax, 0, 2 * sizeof(unsigned int), scomp));  // one entry that every slab raises
   for (int k = 0; k < C; ++k) {
     for (int d = -1; d <= 1; ++d) PMF_CK(cudaStreamWaitEvent(scomp, arrived(((k + d) % C + C) % C), 0));
     StepArgs a;
-    fill_glm_args(a, Ud, Und, nullptr, false, dtdx, ch, decay, c->d_smax);
+    fill_glm_args(a, Ud, Und, nullptr, false, dtdx, ch, decay, c->d_smax + 1);
+    a.smax_part = 0;
     a.zlo = zb(k);
     a.zhi = zb(k + 1);
     if ((rc = launch_step(c, g, a, t, false, false, scomp))) return rc;
@@ -592,8 +653,8 @@ int pmfmhd_max_wavespeed(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const
   cudaStream_t s = as_stream(stream);
   CPtr9 u;
   for (int f = 0; f < 9; ++f) u.p[f] = U[f];
-  PMF_CK(cudaMemsetAsync(c->d_smax, 0, sizeof(unsigned int), s));
-  wavespeed_kernel<<<aux_blocks(c, ncells(g)), AUX_THREADS, 0, s>>>(u, (int)ncells(g), phys_of(g), c->d_smax);
+  const int nb = std::min(aux_blocks(c, ncells(g)), kSmaxMax - 1);
+  wavespeed_kernel<<<nb, AUX_THREADS, 0, s>>>(u, (int)ncells(g), phys_of(g), c->d_smax);
   PMF_CK(cudaGetLastError());
   return read_smax(c, smax, s);
 }
@@ -748,7 +809,6 @@ int pmfmhd_run_glm(pmfmhd_ctx* c, const pmfmhd_grid* g, float* const U[9], float
     float* const* dst = (n % 2 == 0) ? scratch : U;
     StepArgs a;
     fill_glm_args(a, src, dst, resid, comp, dtdx, ch, decay, c->d_smax);
-    cudaMemsetAsync(c->d_smax, 0, sizeof(unsigned int), c->cap);
     int lrc = launch_step(c, g, a, t, false, comp, c->cap);
     if (lrc != PMFMHD_OK) {
       cudaGraph_t dead = nullptr;
@@ -806,9 +866,9 @@ int pmfmhd_autotune(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const U[9]
       result = PMFMHD_ECUDA;
   cudaMemsetAsync(res[0], 0, (size_t)7 * nc * sizeof(float), s);
   if (ct) cudaMemsetAsync(ctp, 0, (size_t)CT_NSLOT * nc * sizeof(float), s);
-  Tune best = default_tune(c, g);
+  Tune best = default_tune(c, g, ct, SRC_NONE);
   float best_ms = 1e30f;
-  std::vector<int> tzs = {8, 32};
+  std::vector<int> tzs = {1, 8};
   for (int ty : kTileRows) {
     if (ty > 5 && g->ny < ty) continue;
     for (int tz : tzs) {
@@ -860,7 +920,6 @@ int pmfmhd_step_glm_census(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* con
   StepArgs a;
   fill_glm_args(a, U, Unew, nullptr, false, dt / g->dx, ch, decay, c->d_smax);
   a.census = cnt;
-  PMF_CK(cudaMemsetAsync(c->d_smax, 0, sizeof(unsigned int), s));
   Tune t = tune_for(c, g, false, false);
   t.ty = kCensusRows;
   const StepKernelInfo k = step_census_kernel_info();

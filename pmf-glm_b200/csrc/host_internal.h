@@ -78,7 +78,7 @@ struct HostPath {
 struct pmfmhd_ctx {
   int device = 0;
   int sms = 148;
-  unsigned int* d_smax = nullptr;           // bits of the last step's max signal speed
+  unsigned int* d_smax = nullptr;           // the last step's max signal speeds: a count, then bits per CTA
   unsigned long long* d_u64 = nullptr;      // bits of an FP64 max
   double* d_partial = nullptr;              // totals partials
   double* d_tot = nullptr;                  // totals
@@ -97,7 +97,8 @@ struct pmfmhd_ctx {
 
 namespace pmf {
 namespace host {
-Tune tune_for(pmfmhd_ctx* c, const pmfmhd_grid* g, bool ct, bool comp);
+Tune tune_for(pmfmhd_ctx* c, const pmfmhd_grid* g, bool ct, bool comp, int src = 0);
+Tune batch_tune(pmfmhd_ctx* c, const pmfmhd_grid* g, bool ct, bool comp);
 // Tensor maps for the nine fields U (box PLANE_W x (ty+4) x 1); false if TMA cannot be used
 // for this grid (x extent not a multiple of 4, unaligned pointers, box larger than the grid).
 bool field_maps(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const U[9], int ty, CUtensorMap out[9]);

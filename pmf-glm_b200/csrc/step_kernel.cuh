@@ -75,6 +75,9 @@ struct StepArgs {
   float dtdx, ch, decay;
   Phys P;
   unsigned int* smax_bits;  // fused CFL reduction target (bits of a non-negative float), or null
+  int smax_part;            // smax_bits is an array: CTA b stores its maximum in entry b + 1 and entry 0
+                            // holds the CTAs less one (nothing to clear beforehand); 0: one cell,
+                            // cleared by the caller, that the CTAs raise
   const float* dscal;       // if non-null: device {dtdx, ch, decay} overriding the values above
   unsigned int* status;     // device status bits (1: a bounded wait for a TMA load gave up), or null
   int use_tma;              // the tensor maps below describe U (fields with nx % 4 == 0)
@@ -85,6 +88,8 @@ struct StepArgs {
   CUtensorMap tmap[9];      // per field: 3-D (x, y, z) FP32 map, box (PLANE_W, TY+4, 1)
   DragCoef drag;            // source-coupled steps: drag coefficients (read by SRC_DRAG/SRC_RAD kernels)
   int zlo, zhi;             // single-box launches: the planes [zlo, zhi) this launch updates
+  int zparts;               // > 0: each column's planes are cut into this many equal parts, one per CTA;
+                            // 0: the CTAs share the (column, plane) space evenly (cta_range)
   float* corr;              // SRC_RAD: packed 9*nc correction buffer (slot 0 psi, 1-3 velocity
                             // corrections, 4 density increments, 5-7 B / 8 E remainders)
   int rad_flags;            // SRC_RAD: RAD_* bits
@@ -176,7 +181,11 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // One column segment: planes [z0, z1) of column tile (tx, ty) of the box described by `a`.
 // Every thread of the CTA calls it; `smax` accumulates the new state's max signal speed.
 // TMA: the instantiation carries the bulk-tensor staging path (used where a.use_tma is set).
-template <int TY, int RECON, int RSOL, bool CT, bool COMP, int SRC, bool TMA>
+// PROLOGUE: the segment's first three planes are staged by code of their own instead of by passes
+// of the plane loop that do nothing else. The batched kernel wants it (the 64-box mix 6.71 -> 6.33
+// ms per two steps; without it the kernel sits at its register cap); in the single-box kernel
+// it only repeats code that a small box then has to fetch (64^3 37.9 against 38.7 us).
+template <int TY, int RECON, int RSOL, bool CT, bool COMP, int SRC, bool TMA, bool PROLOGUE>
 __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, int z0, int z1, float* smem,
                                              float& smax, unsigned long long* tma_bar, unsigned& tma_phase,
                                              int* tma_off, HlldCensus& cz) {
@@ -259,9 +268,9 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
   const unsigned bar_addr = (unsigned)__cvta_generic_to_shared(tma_bar);
   auto issue_plane = [&](int zp) {  // loaders only
     pending_tma = false;
-    if (*tma_off != 0) return;  // degraded staging: convert_plane reads global memory
+    if (TMA && *tma_off != 0) return;  // degraded staging: convert_plane reads global memory
     pending_tma = tma_cols && zp >= 0 && zp < nz;
-    if (pending_tma) {
+    if (TMA && pending_tma) {
       if (lt == 0) {
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar_addr),
@@ -299,7 +308,7 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
   // result is still the step's.
   const int poll_limit = a.tma_stall_polls > 0 ? a.tma_stall_polls : (1 << 22);
   auto wait_plane = [&]() {
-    if (!pending_tma) {
+    if (!TMA || !pending_tma) {
       cp_async_wait_all();
       return;
     }
@@ -351,34 +360,36 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
     }
   };
   auto convert_plane = [&](int zp, float* dst) {
-    if (*tma_off != 0) convert_from(std::true_type{}, zp, dst);
+    if (TMA && *tma_off != 0) convert_from(std::true_type{}, zp, dst);
     else convert_from(std::false_type{}, zp, dst);
   };
   // barrier among the loader warps only (named barrier 1)
   auto loader_sync = [&]() { asm volatile("bar.sync 1, %0;\n" ::"r"(S::NL) : "memory"); };
-  auto slot = [&](int zp) { return prim + ((zp - z0 + 4) & 3) * (9 * S::PPC); };
+  auto slot = [&](int zp) { return prim + ((zp - z0 + 4) & 3) * (9 * S::PPC); };  // zp >= z0 - 2
   auto ld9 = [&](const float* pl, int r, int c) { return ld9p<S::PPC>(pl, r * S::PRW + c); };
 
   // Prologue: primitives of planes z0-2, z0-1 and z0, plane z0+1 in flight.
-  __syncthreads();  // the previous segment may still be reading shared memory
-  if (loader) {
-    if constexpr (DSTAGE) {
-      issue_plane(z0 - 2);
-      for (int zp = z0 - 2; zp <= z0; ++zp) {
-        wait_plane();
-        loader_sync();
-        issue_plane(zp + 1);  // into the other buffer; zp + 1 <= z0 + 1 <= z1 + 1
-        convert_plane(zp, slot(zp));
+  if constexpr (PROLOGUE) {
+    __syncthreads();  // the previous segment may still be reading shared memory
+    if (loader) {
+      if constexpr (DSTAGE) {
+        issue_plane(z0 - 2);
+        for (int zp = z0 - 2; zp <= z0; ++zp) {
+          wait_plane();
+          loader_sync();
+          issue_plane(zp + 1);  // into the other buffer; zp + 1 <= z0 + 1 <= z1 + 1
+          convert_plane(zp, slot(zp));
+        }
+      } else {
+        for (int zp = z0 - 2; zp <= z0; ++zp) {
+          issue_plane(zp);
+          wait_plane();
+          loader_sync();
+          convert_plane(zp, slot(zp));
+          loader_sync();
+        }
+        if (z0 + 1 <= z1 + 1) issue_plane(z0 + 1);
       }
-    } else {
-      for (int zp = z0 - 2; zp <= z0; ++zp) {
-        issue_plane(zp);
-        wait_plane();
-        loader_sync();
-        convert_plane(zp, slot(zp));
-        loader_sync();
-      }
-      if (z0 + 1 <= z1 + 1) issue_plane(z0 + 1);
     }
   }
 
@@ -396,12 +407,12 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
 
   // radiation: in-plane offset of this thread's cell, wrapped periodically (halo cells and
   // the columns/rows of a partial tile beyond the grid are periodic images)
-  const int rad_xy = RAD ? (((y % ny) + ny) % ny) * nx + ((x % nx) + nx) % nx : 0;
+  const int rad_xy = RAD ? wrap_index(y, ny) * nx + wrap_index(x, nx) : 0;
   // masked fallback: the in-plane offsets of the cells on the lower x and y sides of this
   // cell's lower faces (periodic images), and the mask of this cell in the previous plane
   const bool masked = RAD && (a.rad_flags & RAD_MASKED) != 0;
-  const int rad_xm = RAD ? (((y % ny) + ny) % ny) * nx + (((x - 1) % nx) + nx) % nx : 0;
-  const int rad_ym = RAD ? ((((y - 1) % ny) + ny) % ny) * nx + ((x % nx) + nx) % nx : 0;
+  const int rad_xm = RAD ? wrap_index(y, ny) * nx + wrap_index(x - 1, nx) : 0;
+  const int rad_ym = RAD ? wrap_index(y - 1, ny) * nx + wrap_index(x, nx) : 0;
 
   // Where the register budget allows (TY = 8, 9: three warps per sub-partition), the state and
   // Kahan remainders of the next plane this thread updates are loaded one pass ahead, so their
@@ -488,7 +499,9 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
   bool m_zlo = false;  // mask of this cell in plane p-1 (the lower side of its z-face)
 
   F9 Fx;  // this thread's lower x-face flux of the last owned plane solved
-  for (int p = z0 - 1; p <= z1; ++p) {
+  // Without a prologue the passes p = z0-5 .. z0-2 fill the pipeline: the loaders issue plane p+3
+  // and convert plane p+2 in the code of the regular passes.
+  for (int p = PROLOGUE ? z0 - 1 : z0 - 5; p <= z1; ++p) {
     __syncthreads();  // plane p+1 (converted during the previous pass) is in the ring; the x/y
                       // fluxes of plane p-1 are complete
     // x/y flux divergence of plane p-1 for the owned rows, parked for its update in the z-solve
@@ -511,7 +524,7 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
     float bnx = 0.0f, bny = 0.0f, bnz = 0.0f;
     bool m_c = false;  // masked fallback: this cell of plane p is masked
     // planes z0-1 and z1 only feed the chunk's end z-faces: only the owned rows work on them
-    if (mid || row_own) {
+    if (mid || (row_own && p >= z0 - 1)) {
 
     // CT: the staggered normal fields of this cell's three lower faces, fetched now so that
     // their latency overlaps the Hancock step (x: all solving lanes; y: rows 1..TY+1; z:
@@ -622,15 +635,16 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
     }  // mid || row_own
     // ---- loaders: convert plane p+2 (its ring slot last held p-2) and prefetch p+3 -----------
     if (loader && p + 2 <= z1 + 1) {
-      wait_plane();
+      const bool conv = PROLOGUE || p + 2 >= z0 - 2;
+      if (conv) wait_plane();
       loader_sync();
       if constexpr (DSTAGE) {
         // the other buffer was last read by convert(p+1), which every loader finished before
         // this barrier
         if (p + 3 <= z1 + 1) issue_plane(p + 3);
-        convert_plane(p + 2, slot(p + 2));
+        if (conv) convert_plane(p + 2, slot(p + 2));
       } else {
-        convert_plane(p + 2, slot(p + 2));
+        if (conv) convert_plane(p + 2, slot(p + 2));
         loader_sync();
         if (p + 3 <= z1 + 1) issue_plane(p + 3);
       }
@@ -725,9 +739,10 @@ __device__ __forceinline__ void init_tma_barrier(unsigned long long* bar, int* o
   __syncthreads();
 }
 
-// Block-wide max of v and one atomicMax into *bits (every thread of the CTA calls it).
+// Block-wide max of v: one atomicMax into *bits, or (part) stored as this CTA's entry of the array
+// `bits` (every thread of the CTA calls it).
 template <int NT>
-__device__ __forceinline__ void flush_smax(float v, unsigned int* bits) {
+__device__ __forceinline__ void flush_smax(float v, unsigned int* bits, bool part = false) {
   __shared__ float red[32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   __syncthreads();
@@ -737,7 +752,14 @@ __device__ __forceinline__ void flush_smax(float v, unsigned int* bits) {
   if (w == 0) {
     v = lane < NT / 32 ? red[lane] : 0.0f;
     v = warp_max(v);
-    if (lane == 0) atomicMax(bits, __float_as_uint(v));
+    if (lane == 0) {
+      if (!part) {
+        atomicMax(bits, __float_as_uint(v));
+      } else {
+        bits[blockIdx.x + 1] = __float_as_uint(v);
+        if (blockIdx.x == 0) bits[0] = gridDim.x - 1;
+      }
+    }
   }
 }
 
@@ -749,10 +771,10 @@ __device__ __forceinline__ void cta_range(long long Q, long long* q0, long long*
   *q1 = Q * (blockIdx.x + 1) / gridDim.x;
 }
 
-// One box: a persistent launch of one CTA per resident slot. The plain and compensated GLM
-// instantiations stage interior planes by TMA; the CT and source-coupled ones are compiled
-// without the TMA path and stage every plane by cp.async: the path's code cost them 4 % (CT,
-// 2.38 against 2.29 ms per 256^3 step), 2 % (drag) and 5 % (radiation), the GLM step 0.5 %.
+// One box: a persistent launch of one CTA per resident slot. The plain GLM instantiations stage
+// interior planes by TMA; the others are compiled without the TMA path and stage every plane by
+// cp.async: the path's code cost the compensated step 6 % (256^3, 1.66 against 1.57 ms), CT 4 %,
+// the drag-coupled step 2 % and the radiation-coupled one 5 %; of the plain step it is 0.5-1 %.
 template <int TY, int RECON, int RSOL, bool CT, bool COMP, int SRC>
 __global__ void __launch_bounds__(step_threads<TY>(), step_min_blocks<TY>()) mhd_step_kernel(const __grid_constant__ StepArgs a) {
   extern __shared__ __align__(128) float smem[];
@@ -762,7 +784,13 @@ __global__ void __launch_bounds__(step_threads<TY>(), step_min_blocks<TY>()) mhd
   init_tma_barrier(&tma_bar, &tma_off);
   long long q, qe;
   const int nzr = a.zhi - a.zlo;  // planes of this launch
-  cta_range((long long)a.ntx * a.nty * nzr, &q, &qe);
+  if (a.zparts > 0) {
+    const int col = (int)blockIdx.x / a.zparts, part = (int)blockIdx.x - col * a.zparts;
+    q = (long long)col * nzr + (long long)nzr * part / a.zparts;
+    qe = (long long)col * nzr + (long long)nzr * (part + 1) / a.zparts;
+  } else {
+    cta_range((long long)a.ntx * a.nty * nzr, &q, &qe);
+  }
   float smax = 0.0f;
   HlldCensus cz{0u, 0u, 0u};
   while (q < qe) {
@@ -770,14 +798,14 @@ __global__ void __launch_bounds__(step_threads<TY>(), step_min_blocks<TY>()) mhd
     const int zr = (int)(q - (long long)col * nzr);
     const int z0 = a.zlo + zr;
     const int z1 = a.zlo + (int)min((long long)nzr, zr + (qe - q));
-    march_column<TY, RECON, RSOL, CT, COMP, SRC, !CT && SRC == SRC_NONE>(a, col % a.ntx, col / a.ntx, z0, z1, smem, smax, &tma_bar,
+    march_column<TY, RECON, RSOL, CT, COMP, SRC, !CT && !COMP && SRC == SRC_NONE, false>(a, col % a.ntx, col / a.ntx, z0, z1, smem, smax, &tma_bar,
                                                   tma_phase, &tma_off, cz);
     q += z1 - z0;
   }
   drain_tma(&tma_bar, tma_phase, &tma_off, a.tma_stall_polls > 0 ? a.tma_stall_polls : (1 << 22),
             step_stage_lead<TY>());
   if constexpr (RSOL == RS_HLLD_CENSUS) flush_census(cz, a.census);
-  if (!CT && a.smax_bits != nullptr) flush_smax<step_threads<TY>()>(smax, a.smax_bits);
+  if (!CT && a.smax_bits != nullptr) flush_smax<step_threads<TY>()>(smax, a.smax_bits, a.smax_part != 0);
 }
 
 // Many boxes in one launch: box b owns global indices [q0_b, q0_{b+1}) of the concatenated
@@ -819,7 +847,7 @@ __global__ void __launch_bounds__(step_threads<TY>(), step_min_blocks<TY>()) mhd
     const int col = (int)(local / a.nz);
     const int z0 = (int)(local - (long long)col * a.nz);
     const int z1 = (int)min((long long)a.nz, z0 + (qe - q));
-    march_column<TY, RECON, RSOL, CT, COMP, SRC_NONE, false>(a, col % a.ntx, col / a.ntx, z0, z1, smem, smax, &tma_bar,
+    march_column<TY, RECON, RSOL, CT, COMP, SRC_NONE, false, true>(a, col % a.ntx, col / a.ntx, z0, z1, smem, smax, &tma_bar,
                                                    tma_phase, &tma_off, cz);
     q += z1 - z0;
   }
