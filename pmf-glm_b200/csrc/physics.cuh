@@ -115,18 +115,6 @@ __device__ __forceinline__ float minmod(float dl, float dr) {
   float sgn = dl >= 0.0f ? 1.0f : -1.0f;
   return dl * dr <= 0.0f ? 0.0f : sgn * fminf(fabsf(dl), fabsf(dr));
 }
-// local CW84 PPM edges, monotonised (glm_physics.jl:188-200)
-__device__ __forceinline__ void ppm_edges(float qm, float q0, float qp, float& oL, float& oR) {
-  float slope = (qp - qm) * 0.25f;
-  float curve = (qm - 2.0f * q0 + qp) / 12.0f;
-  float qL = q0 - slope + curve, qR = q0 + slope + curve, qa = q0;
-  float dq = qR - qL, qmid = 0.5f * (qL + qR), dq2_6 = dq * dq / 6.0f, diff = (qa - qmid) * dq;
-  if ((qR - qa) * (qa - qL) <= 0.0f) { oL = qa; oR = qa; }
-  else if (diff > dq2_6) { oL = 3.0f * qa - 2.0f * qR; oR = qR; }
-  else if (diff < -dq2_6) { oL = qL; oR = 3.0f * qa - 2.0f * qL; }
-  else { oL = qL; oR = qR; }
-}
-
 // Per-axis face offsets about the cell mean. For the PLM limiters dL = -dR, so only dR is
 // produced and dL is implied (glm_physics.jl:212-219); PPM produces both (:220-223).
 template <int RECON> struct Offsets {
@@ -165,6 +153,23 @@ __device__ __forceinline__ float min_xorsign_abs(float a, float b) {
 __device__ __forceinline__ float half_moncen(float dl, float dr, float q) {
   return min_xorsign_abs(fmaxf(min_xorsign_abs(dl, dr), 0.0f), q);
 }
+// Local CW84 PPM face offsets, monotonised (glm_physics.jl:188-200), from the differences to the
+// lower and upper neighbour. Before the limiter the offsets are L = c - s, R = c + s with
+// s = (dl + dr)/4, c = (dr - dl)/12. The reference's cases are: L and R on the same side (an
+// extremum): both zero; (q - mid)(R - L) > (R - L)^2/6, that is |L| > 2|R|: L = -2R; likewise
+// R = -2L; otherwise unchanged. That is |L| and |R| cut at twice the smaller of the two, or at
+// zero where their signs agree: z = max(-min.xorsign(L, R), 0) is that smaller magnitude or
+// zero. No branch and no division (the reference's form diverges within a warp and divides
+// twice a field: the 192^3 PPM/HLLD step took 1.39 ms with it, 0.73 with this form and the
+// solver above).
+__device__ __forceinline__ void ppm_offsets(float dl, float dr, float& oL, float& oR) {
+  const float s = 0.25f * (dl + dr), c = dr - dl;
+  const float L = fmaf(1.0f / 12.0f, c, -s), R = fmaf(1.0f / 12.0f, c, s);
+  const float z2 = 2.0f * fmaxf(-min_xorsign_abs(L, R), 0.0f);
+  oL = min_xorsign_abs(L, z2);
+  oR = min_xorsign_abs(R, z2);
+}
+
 template <int RECON>
 __device__ __forceinline__ Offsets<RECON> recon(const F9& mm, const F9& m0, const F9& mp) {
   Offsets<RECON> o;
@@ -180,10 +185,7 @@ __device__ __forceinline__ Offsets<RECON> recon(const F9& mm, const F9& m0, cons
   } else {
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
-      float a, b;
-      ppm_edges(mm[i], m0[i], mp[i], a, b);
-      o.dL[i] = a - m0[i];
-      o.dR[i] = b - m0[i];
+      ppm_offsets(m0[i] - mm[i], mp[i] - m0[i], o.dL[i], o.dR[i]);
     }
   }
   return o;
