@@ -339,7 +339,9 @@ __device__ __forceinline__ float ct_bcc_col(const float* __restrict__ bxf, const
   return m;
 }
 
-static __global__ void __launch_bounds__(AUX_THREADS) ct_emf_col_kernel(
+// Four blocks an SM: left alone the kernel takes 80 registers, three blocks, and had too few
+// loads in flight (256^3: 246 us, 195 with 64 registers).
+static __global__ void __launch_bounds__(AUX_THREADS, 4) ct_emf_col_kernel(
     const float* __restrict__ MFX, const float* __restrict__ MFY, const float* __restrict__ MFZ,
     const float* __restrict__ FXBY, const float* __restrict__ FXBZ, const float* __restrict__ FYBX,
     const float* __restrict__ FYBZ, const float* __restrict__ FZBX, const float* __restrict__ FZBY,
