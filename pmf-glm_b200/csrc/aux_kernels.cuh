@@ -111,6 +111,61 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb_kernel(const float* _
   if (threadIdx.x == 0) atomicMax(out_bits, (unsigned long long)__double_as_longlong(m * inv2dx));
 }
 
+// The same with four cells of a row per lane (fields 16-byte aligned, nx a multiple of 4): the
+// scalar form executes 144 instructions a cell and warp, most of them for its indices, and takes
+// 119 us at 256^3, four times its traffic.
+static __global__ void __launch_bounds__(AUX_THREADS) divb4_kernel(const float* __restrict__ bx, const float* __restrict__ by,
+                                                            const float* __restrict__ bz, int nx, int ny, int nz, int zc,
+                                                            int bcx, int bcy, int bcz, double inv2dx,
+                                                            unsigned long long* out_bits) {
+  const int ti = (blockIdx.x * COL_X + (threadIdx.x & 31)) * 4, tj = blockIdx.y * COL_Y + (threadIdx.x >> 5);
+  const bool in = ti < nx && tj < ny;
+  const int i = min(ti, nx - 4), j = min(tj, ny - 1);
+  float fxp, fxm, fyp, fym, fzm, fzp;
+  const unsigned row = (unsigned)j * nx;
+  const unsigned oxp = row + bc_index(i + 4, nx, bcx, &fxp), oxm = row + bc_index(i - 1, nx, bcx, &fxm);
+  const unsigned oyp = (unsigned)bc_index(j + 1, ny, bcy, &fyp) * nx + i;
+  const unsigned oym = (unsigned)bc_index(j - 1, ny, bcy, &fym) * nx + i;
+  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
+  const size_t nxy = (size_t)nx * ny;
+  const float* top = bz + bc_index(nz, nz, bcz, &fzp) * nxy + row + i;  // the plane above the last
+  double m = 0.0;
+  float lo = __double2float_rd(__longlong_as_double(*(volatile long long*)out_bits) / inv2dx * (1.0 - 1e-6));
+  auto ld4 = [](const float* p) { return *reinterpret_cast<const float4*>(p); };
+  auto mul4 = [](float4 v, float f) { return make_float4(v.x * f, v.y * f, v.z * f, v.w * f); };
+  const size_t below = bc_index(z0 - 1, nz, bcz, &fzm) * nxy;
+  float4 zm = mul4(ld4(bz + below + row + i), fzm);
+  const float *xr = bx + z0 * nxy, *yr = by + z0 * nxy, *zr = bz + z0 * nxy + row + i;
+  float4 z = ld4(zr);
+  for (int k = z0; k < z1; ++k, xr += nxy, yr += nxy, zr += nxy) {
+    const float4 zp = k + 1 == nz ? mul4(ld4(top), fzp) : ld4(zr + nxy);
+    const float4 c = ld4(xr + row + i), yp = mul4(ld4(yr + oyp), fyp), ym = mul4(ld4(yr + oym), fym);
+    const float xl = xr[oxm] * fxm, xu = xr[oxp] * fxp;
+    const float xp[4] = {c.y, c.z, c.w, xu}, xm[4] = {xl, c.x, c.y, c.z};
+    const float ypa[4] = {yp.x, yp.y, yp.z, yp.w}, yma[4] = {ym.x, ym.y, ym.z, ym.w};
+    const float zpa[4] = {zp.x, zp.y, zp.z, zp.w}, zma[4] = {zm.x, zm.y, zm.z, zm.w};
+    float reach = 0.0f;  // the largest the four may be
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float d = (xp[q] - xm[q]) + (ypa[q] - yma[q]) + (zpa[q] - zma[q]);
+      const float mag = fabsf(xp[q]) + fabsf(xm[q]) + fabsf(ypa[q]) + fabsf(yma[q]) + fabsf(zpa[q]) + fabsf(zma[q]);
+      reach = fmaxf(reach, fmaf(4.7683716e-7f, mag, fabsf(d)));  // 2^-21 mag
+    }
+    const bool maybe = in && reach >= lo;
+    if (maybe) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        m = fmax(m, fabs((double)xp[q] - (double)xm[q] + (double)ypa[q] - (double)yma[q] + (double)zpa[q] - (double)zma[q]));
+      lo = fmaxf(lo, __double2float_rd(m));
+    }
+    if (__any_sync(0xffffffffu, maybe)) lo = warp_max(lo);
+    zm = z;
+    z = zp;
+  }
+  m = block_reduce_max(m);
+  if (threadIdx.x == 0) atomicMax(out_bits, (unsigned long long)__double_as_longlong(m * inv2dx));
+}
+
 // max face divergence of a CT face field, FP64 (ct.jl:176-185)
 static __global__ void __launch_bounds__(AUX_THREADS) divb_face_kernel(const float* __restrict__ bxf,
                                                                 const float* __restrict__ byf,
@@ -180,6 +235,7 @@ static __global__ void __launch_bounds__(AUX_THREADS) totals_final_kernel(const 
                                                                    double* out) {
   __shared__ double red[AUX_THREADS];
   double t = 0.0;
+#pragma unroll 16
   for (int b = threadIdx.x >> 3; b < nblocks; b += AUX_THREADS / 8) t += partial[b * 8 + (threadIdx.x & 7)];
   red[threadIdx.x] = t;
   for (int n = AUX_THREADS / 2; n >= 8; n >>= 1) {
