@@ -180,11 +180,14 @@ def context(device: Optional[int] = None):
 
 
 def _stream():
-    return _VP(torch.cuda.current_stream().cuda_stream)
+    # the raw handle: a torch.cuda.Stream object costs as much host time as the launch itself
+    return _VP(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _p9(ts) -> "ctypes.Array":
-    return _P9(*[t.data_ptr() for t in ts])
+    a = _P9()
+    a[:] = [t.data_ptr() for t in ts]  # a third of the time of passing nine arguments
+    return a
 
 
 @dataclass
