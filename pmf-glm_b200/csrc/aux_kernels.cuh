@@ -38,6 +38,8 @@ template <class T> __device__ __forceinline__ T block_reduce_max(T v) {
 // the blocks less one in out_bits[0]
 static __global__ void __launch_bounds__(AUX_THREADS) wavespeed_kernel(const CPtr9 U, int nc, Phys P,
                                                                 unsigned int* out_bits) {
+  overlap_next();
+  wait_previous();
   float m = 0.0f;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
     F9 u;
@@ -404,6 +406,8 @@ static __global__ void __launch_bounds__(AUX_THREADS, 4) ct_emf_col_kernel(
     const float* __restrict__ ECX, const float* __restrict__ ECY, const float* __restrict__ ECZ,
     float* __restrict__ EX, float* __restrict__ EY, float* __restrict__ EZ, int nx, int ny, int nz,
     int zc, unsigned int* __restrict__ smax) {
+  overlap_next();
+  wait_previous();
   // the signal-speed cell that ct_bcc_col_kernel raises two launches later: one entry, 0
   if (threadIdx.x < 2 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) smax[threadIdx.x] = 0u;
   ct_emf_col(MFX, MFY, MFZ, FXBY, FXBZ, FYBX, FYBZ, FZBX, FZBY, ECX, ECY, ECZ, EX, EY, EZ, nx, ny, nz, blockIdx.x,
@@ -415,12 +419,16 @@ static __global__ void __launch_bounds__(AUX_THREADS) ct_face_col_kernel(
     const float* __restrict__ ex, const float* __restrict__ ey, const float* __restrict__ ez,
     float* __restrict__ bxf, float* __restrict__ byf, float* __restrict__ bzf, float* __restrict__ rbx,
     float* __restrict__ rby, float* __restrict__ rbz, int nx, int ny, int nz, int zc, float dtdx) {
+  overlap_next();
+  wait_previous();
   ct_face_col<COMP>(ex, ey, ez, bxf, byf, bzf, rbx, rby, rbz, nx, ny, nz, dtdx, blockIdx.x, blockIdx.y, blockIdx.z, zc);
 }
 
 static __global__ void __launch_bounds__(AUX_THREADS) ct_bcc_col_kernel(
     const float* __restrict__ bxf, const float* __restrict__ byf, const float* __restrict__ bzf, const MPtr9 Un,
     int nx, int ny, int nz, int zc, Phys P, unsigned int* smax_bits) {
+  overlap_next();
+  wait_previous();
   float m = ct_bcc_col(bxf, byf, bzf, Un, nx, ny, nz, P, smax_bits != nullptr, blockIdx.x, blockIdx.y, blockIdx.z, zc);
   if (smax_bits != nullptr) {
     m = block_reduce_max(m);

@@ -220,9 +220,43 @@ int occupancy_of(const StepKernelInfo& k) {
   return occ;
 }
 
+// Whether a box's launches overlap the previous kernel of the stream (overlap_next / wait_previous in
+// the kernels): the launch latency, some 2 us a kernel, is then hidden behind that kernel's tail
+// (32^3 GLM step 16.4 -> 14.1 us, 48^3 CT 39.8 -> 32.4, 128^3 CT 275 -> 270). Past about 160^3 cells
+// it is nothing beside the kernels, whose last CTAs the early CTAs then disturb (256^3 CT 1.957
+// -> 1.967 ms).
+bool overlaps(const pmfmhd_grid* g) { return ncells(g) <= (1LL << 22); }
+
+cudaError_t launch_kernel(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t s,
+                          bool overlap) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelExC(&cfg, fn, args);
+}
+// A companion kernel of AUX_THREADS threads per block on `grid` blocks.
+template <class... P, class... A>
+cudaError_t launch_aux(void (*fn)(P...), dim3 grid, cudaStream_t s, bool overlap, A... a) {
+  std::tuple<P...> p(a...);
+  return std::apply(
+      [&](P&... v) {
+        void* args[] = {(void*)&v...};
+        return launch_kernel((const void*)fn, grid, dim3(AUX_THREADS), args, 0, s, overlap);
+      },
+      p);
+}
+
+// `overlap`: the launch may overlap the previous kernel of the stream (if the box is small enough).
 // `force`: launch this instantiation (its tile height in t.ty) instead of the dispatched one.
 int launch_step(pmfmhd_ctx* c, const pmfmhd_grid* g, StepArgs& a, Tune t, bool ct, bool comp,
-                cudaStream_t s, int src = SRC_NONE, const StepKernelInfo* force = nullptr) {
+                cudaStream_t s, int src = SRC_NONE, bool overlap = true, const StepKernelInfo* force = nullptr) {
   StepKernelInfo k = force ? *force : step_kernel_info(t.ty, g->recon, g->riemann, ct, comp, src);
   if (k.fn == nullptr) return PMFMHD_EUNSUPPORTED;
   const int occ = occupancy_of(k);
@@ -245,7 +279,8 @@ int launch_step(pmfmhd_ctx* c, const pmfmhd_grid* g, StepArgs& a, Tune t, bool c
   a.zparts = sp.zparts;
   const int blocks = sp.blocks;
   void* args[] = {(void*)&a};
-  PMF_CK(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)blocks), dim3(k.threads), args, k.smem_bytes, s));
+  PMF_CK(launch_kernel((const void*)k.fn, dim3((unsigned)blocks), dim3(k.threads), args, k.smem_bytes, s,
+                       overlap && overlaps(g)));
   return PMFMHD_OK;
 }
 
@@ -329,23 +364,17 @@ int enqueue_ct(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const U[9], flo
   auto sl = [&](int k) { return ct + (size_t)k * nc; };
   int zc;
   const dim3 cg = ctc_grid(g->nx, g->ny, g->nz, c->sms, &zc);
-  ct_emf_col_kernel<<<cg, AUX_THREADS, 0, s>>>(sl(CT_MFX), sl(CT_MFY), sl(CT_MFZ), sl(CT_FXBY), sl(CT_FXBZ),
-                                               sl(CT_FYBX), sl(CT_FYBZ), sl(CT_FZBX), sl(CT_FZBY), sl(CT_ECX),
-                                               sl(CT_ECY), sl(CT_ECZ), sl(CT_EX), sl(CT_EY), sl(CT_EZ), g->nx,
-                                               g->ny, g->nz, zc, c->d_smax);
-  if (comp_faces)
-    ct_face_col_kernel<true><<<cg, AUX_THREADS, 0, s>>>(sl(CT_EX), sl(CT_EY), sl(CT_EZ), sl(CT_BXF), sl(CT_BYF),
-                                                        sl(CT_BZF), sl(CT_RBX), sl(CT_RBY), sl(CT_RBZ), g->nx, g->ny, g->nz,
-                                                        zc, dtdx);
-  else
-    ct_face_col_kernel<false><<<cg, AUX_THREADS, 0, s>>>(sl(CT_EX), sl(CT_EY), sl(CT_EZ), sl(CT_BXF), sl(CT_BYF),
-                                                         sl(CT_BZF), sl(CT_RBX), sl(CT_RBY), sl(CT_RBZ), g->nx, g->ny, g->nz,
-                                                        zc, dtdx);
+  const bool ov = overlaps(g);
+  PMF_CK(launch_aux(ct_emf_col_kernel, cg, s, ov, sl(CT_MFX), sl(CT_MFY), sl(CT_MFZ), sl(CT_FXBY), sl(CT_FXBZ),
+                    sl(CT_FYBX), sl(CT_FYBZ), sl(CT_FZBX), sl(CT_FZBY), sl(CT_ECX), sl(CT_ECY), sl(CT_ECZ), sl(CT_EX),
+                    sl(CT_EY), sl(CT_EZ), g->nx, g->ny, g->nz, zc, c->d_smax));
+  PMF_CK(launch_aux(comp_faces ? ct_face_col_kernel<true> : ct_face_col_kernel<false>, cg, s, ov, sl(CT_EX),
+                    sl(CT_EY), sl(CT_EZ), sl(CT_BXF), sl(CT_BYF), sl(CT_BZF), sl(CT_RBX), sl(CT_RBY), sl(CT_RBZ),
+                    g->nx, g->ny, g->nz, zc, dtdx));
   MPtr9 un;
   for (int f = 0; f < 9; ++f) un.p[f] = Un[f];
-  ct_bcc_col_kernel<<<cg, AUX_THREADS, 0, s>>>(sl(CT_BXF), sl(CT_BYF), sl(CT_BZF), un, g->nx, g->ny, g->nz,
-                                               zc, phys_of(g), c->d_smax + 1);
-  PMF_CK(cudaGetLastError());
+  PMF_CK(launch_aux(ct_bcc_col_kernel, cg, s, ov, sl(CT_BXF), sl(CT_BYF), sl(CT_BZF), un, g->nx, g->ny, g->nz, zc,
+                    phys_of(g), c->d_smax + 1));
   return PMFMHD_OK;
 }
 
@@ -526,7 +555,7 @@ int pmfmhd_step_glm_host(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const
     a.smax_part = 0;
     a.zlo = zb(k);
     a.zhi = zb(k + 1);
-    if ((rc = launch_step(c, g, a, t, false, false, scomp))) return rc;
+    if ((rc = launch_step(c, g, a, t, false, false, scomp, SRC_NONE, false))) return rc;
     PMF_CK(cudaEventRecord(computed(k), scomp));
     PMF_CK(cudaStreamWaitEvent(sout, computed(k), 0));
     const size_t off = (size_t)zb(k) * nxy, len = (size_t)(zb(k + 1) - zb(k)) * nxy;
@@ -654,8 +683,7 @@ int pmfmhd_max_wavespeed(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const
   CPtr9 u;
   for (int f = 0; f < 9; ++f) u.p[f] = U[f];
   const int nb = std::min(aux_blocks(c, ncells(g)), kSmaxMax - 1);
-  wavespeed_kernel<<<nb, AUX_THREADS, 0, s>>>(u, (int)ncells(g), phys_of(g), c->d_smax);
-  PMF_CK(cudaGetLastError());
+  PMF_CK(launch_aux(wavespeed_kernel, dim3(nb), s, overlaps(g), u, (int)ncells(g), phys_of(g), c->d_smax));
   return read_smax(c, smax, s);
 }
 
@@ -928,7 +956,7 @@ int pmfmhd_step_glm_census(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* con
   Tune t = tune_for(c, g, false, false);
   t.ty = kCensusRows;
   const StepKernelInfo k = step_census_kernel_info();
-  if ((rc = launch_step(c, g, a, t, false, false, s, SRC_NONE, &k))) return rc;
+  if ((rc = launch_step(c, g, a, t, false, false, s, SRC_NONE, true, &k))) return rc;
   PMF_CK(cudaMemcpyAsync(c->h_pin, cnt, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
   PMF_CK(cudaStreamSynchronize(s));
   unsigned long long v[3];

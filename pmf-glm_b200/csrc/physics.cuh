@@ -593,6 +593,13 @@ __device__ __forceinline__ int bc_index(int i, int n, int code, float* flip) {
   return r < 0 ? 0 : (r >= n ? n - 1 : r);
 }
 
+// Programmatic dependent launch. A kernel that begins with overlap_next() / wait_previous() may be
+// launched with that attribute: its CTAs are placed while the previous kernel of the stream still
+// runs and touch memory only after wait_previous(), which returns when that kernel is complete and
+// its writes are visible. Both do nothing in an ordinary launch.
+__device__ __forceinline__ void overlap_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

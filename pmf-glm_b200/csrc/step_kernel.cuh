@@ -781,7 +781,9 @@ __global__ void __launch_bounds__(step_threads<TY>(), step_min_blocks<TY>()) mhd
   __shared__ unsigned long long tma_bar;
   __shared__ int tma_off;
   unsigned tma_phase = 0;
+  overlap_next();
   init_tma_barrier(&tma_bar, &tma_off);
+  wait_previous();
   long long q, qe;
   const int nzr = a.zhi - a.zlo;  // planes of this launch
   if (a.zparts > 0) {
