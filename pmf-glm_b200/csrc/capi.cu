@@ -117,7 +117,7 @@ Split split_work(long long cols, int nz, long long slots, int tz) {
 
 // Tile height of an untuned grid: the height whose longest CTA takes least, its planes times the
 // relative time of one plane of a full GPU. Measured at 256^3: 3.4, 3.85 us a plane at 8 and 9
-// rows for GLM, 3.5, 4.15 for CT, 6.2, 6.8, 8.9 at 8, 9 and 13 for the radiation-coupled step
+// rows for GLM, 3.5, 4.15 for CT, 5.1, 5.6, 7.6 at 8, 9 and 13 for the radiation-coupled step
 // (which waits on its loads of the correction arrays, so that its 16 warps at 13 rows pay; the
 // others are slower at 13 rows for every size). A grid under 8 rows takes the 5-row tile.
 Tune default_tune(const pmfmhd_ctx* c, const pmfmhd_grid* g, bool ct, int src) {
@@ -126,7 +126,7 @@ Tune default_tune(const pmfmhd_ctx* c, const pmfmhd_grid* g, bool ct, int src) {
     int ty;
     double glm, ct, rad;
   };
-  constexpr Cost kCost[] = {{8, 1.0, 1.0, 1.0}, {9, 1.13, 1.18, 1.09}, {13, 1e9, 1e9, 1.43}};
+  constexpr Cost kCost[] = {{8, 1.0, 1.0, 1.0}, {9, 1.13, 1.18, 1.10}, {13, 1e9, 1e9, 1.50}};
   Tune best{8, 1};
   double least = 1e300;
   for (const Cost& k : kCost) {
