@@ -38,13 +38,13 @@ template <class T> __device__ __forceinline__ T block_reduce_max(T v) {
 // the blocks less one in out_bits[0]
 static __global__ void __launch_bounds__(AUX_THREADS) wavespeed_kernel(const CPtr9 U, int nc, Phys P,
                                                                 unsigned int* out_bits) {
-  overlap_next();
   wait_previous();
+  overlap_next();
   float m = 0.0f;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
     F9 u;
 #pragma unroll
-    for (int f = 0; f < 9; ++f) u[f] = __ldg(U.p[f] + c);
+    for (int f = 0; f < 9; ++f) u[f] = U.p[f][c];
     m = fmaxf(m, cell_wavespeed(u, P));
   }
   m = block_reduce_max(m);
@@ -400,14 +400,14 @@ __device__ __forceinline__ float ct_bcc_col(const float* __restrict__ bxf, const
 // Four blocks an SM: left alone the kernel takes 80 registers, three blocks, and had too few
 // loads in flight (256^3: 246 us, 195 with 64 registers).
 static __global__ void __launch_bounds__(AUX_THREADS, 4) ct_emf_col_kernel(
-    const float* __restrict__ MFX, const float* __restrict__ MFY, const float* __restrict__ MFZ,
-    const float* __restrict__ FXBY, const float* __restrict__ FXBZ, const float* __restrict__ FYBX,
-    const float* __restrict__ FYBZ, const float* __restrict__ FZBX, const float* __restrict__ FZBY,
-    const float* __restrict__ ECX, const float* __restrict__ ECY, const float* __restrict__ ECZ,
-    float* __restrict__ EX, float* __restrict__ EY, float* __restrict__ EZ, int nx, int ny, int nz,
-    int zc, unsigned int* __restrict__ smax) {
-  overlap_next();
+    const float* MFX, const float* MFY, const float* MFZ,
+    const float* FXBY, const float* FXBZ, const float* FYBX,
+    const float* FYBZ, const float* FZBX, const float* FZBY,
+    const float* ECX, const float* ECY, const float* ECZ,
+    float* EX, float* EY, float* EZ, int nx, int ny, int nz,
+    int zc, unsigned int* smax) {
   wait_previous();
+  overlap_next();
   // the signal-speed cell that ct_bcc_col_kernel raises two launches later: one entry, 0
   if (threadIdx.x < 2 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) smax[threadIdx.x] = 0u;
   ct_emf_col(MFX, MFY, MFZ, FXBY, FXBZ, FYBX, FYBZ, FZBX, FZBY, ECX, ECY, ECZ, EX, EY, EZ, nx, ny, nz, blockIdx.x,
@@ -416,19 +416,19 @@ static __global__ void __launch_bounds__(AUX_THREADS, 4) ct_emf_col_kernel(
 
 template <bool COMP>
 static __global__ void __launch_bounds__(AUX_THREADS) ct_face_col_kernel(
-    const float* __restrict__ ex, const float* __restrict__ ey, const float* __restrict__ ez,
-    float* __restrict__ bxf, float* __restrict__ byf, float* __restrict__ bzf, float* __restrict__ rbx,
-    float* __restrict__ rby, float* __restrict__ rbz, int nx, int ny, int nz, int zc, float dtdx) {
-  overlap_next();
+    const float* ex, const float* ey, const float* ez,
+    float* bxf, float* byf, float* bzf, float* rbx,
+    float* rby, float* rbz, int nx, int ny, int nz, int zc, float dtdx) {
   wait_previous();
+  overlap_next();
   ct_face_col<COMP>(ex, ey, ez, bxf, byf, bzf, rbx, rby, rbz, nx, ny, nz, dtdx, blockIdx.x, blockIdx.y, blockIdx.z, zc);
 }
 
 static __global__ void __launch_bounds__(AUX_THREADS) ct_bcc_col_kernel(
-    const float* __restrict__ bxf, const float* __restrict__ byf, const float* __restrict__ bzf, const MPtr9 Un,
+    const float* bxf, const float* byf, const float* bzf, const MPtr9 Un,
     int nx, int ny, int nz, int zc, Phys P, unsigned int* smax_bits) {
-  overlap_next();
   wait_previous();
+  overlap_next();
   float m = ct_bcc_col(bxf, byf, bzf, Un, nx, ny, nz, P, smax_bits != nullptr, blockIdx.x, blockIdx.y, blockIdx.z, zc);
   if (smax_bits != nullptr) {
     m = block_reduce_max(m);

@@ -593,12 +593,16 @@ __device__ __forceinline__ int bc_index(int i, int n, int code, float* flip) {
   return r < 0 ? 0 : (r >= n ? n - 1 : r);
 }
 
-// Programmatic dependent launch. A kernel that begins with overlap_next() / wait_previous() may be
+// Programmatic dependent launch. A kernel that begins with wait_previous() / overlap_next() may be
 // launched with that attribute: its CTAs are placed while the previous kernel of the stream still
 // runs and touch memory only after wait_previous(), which returns when that kernel is complete and
-// its writes are visible. Both do nothing in an ordinary launch.
-__device__ __forceinline__ void overlap_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// its writes are visible. overlap_next() comes after the wait, so that the kernel after this one is
+// not placed before the one before this one is complete. Such a kernel is resident while its inputs
+// are written: it reads them by ordinary loads, never through the non-coherent path (no __ldg, no
+// const __restrict__ kernel parameters), whose data must not change while the kernel is resident.
+// Both do nothing in an ordinary launch.
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void overlap_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll

@@ -351,7 +351,7 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
         if constexpr (DIRECT) {
           const int gi = kz * nxy + sidx[(2 * k) * S::NL + lt];
 #pragma unroll
-          for (int f = 0; f < 9; ++f) u[f] = __ldg(a.U[f] + gi);
+          for (int f = 0; f < 9; ++f) u[f] = a.U[f][gi];
         } else {
 #pragma unroll
           for (int f = 0; f < 9; ++f) u[f] = src[f * PP + e];
@@ -431,7 +431,7 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
   auto prefetch_cell = [&](int pz) {
     const int c = pz * nxy + y * nx + x;
 #pragma unroll
-    for (int f = 0; f < 9; ++f) u0[f] = __ldg(a.U[f] + c);
+    for (int f = 0; f < 9; ++f) u0[f] = a.U[f][c];
     if constexpr (COMP) {
 #pragma unroll
       for (int i = 0; i < NR; ++i) rk[i] = a.resid[i][c];
@@ -498,10 +498,10 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
   // x, y and pz are at most one period outside the box, so one conditional wrap suffices.
   auto wrap1 = [](int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); };
   auto face_bn = [&](int D, int pz) {
-    return __ldg(a.face[D] + wrap1(pz, nz) * nxy + wrap1(y, ny) * nx + wrap1(x, nx));
+    return a.face[D][wrap1(pz, nz) * nxy + wrap1(y, ny) * nx + wrap1(x, nx)];
   };
   // fallback mask of in-plane offset xy in plane pz (periodic: pz is at most one period out)
-  auto mask_at = [&](int pz, int xy) { return __ldg(a.mask + (size_t)wrap1(pz, nz) * nxy + xy) > 0.0f; };
+  auto mask_at = [&](int pz, int xy) { return a.mask[(size_t)wrap1(pz, nz) * nxy + xy] > 0.0f; };
   bool m_zlo = false;  // mask of this cell in plane p-1 (the lower side of its z-face)
 
   F9 Fx;  // this thread's lower x-face flux of the last owned plane solved
@@ -601,9 +601,9 @@ __device__ __forceinline__ void march_column(const StepArgs& a, int tx, int ty, 
       if (!halo_warp || halo_act) {
         const size_t n = (size_t)nxy * nz;
         const size_t gi = (size_t)wrap1(p, nz) * nxy + rad_xy;
-        mh[1] += __ldg(a.corr + n + gi);
-        mh[2] += __ldg(a.corr + 2 * n + gi);
-        mh[3] += __ldg(a.corr + 3 * n + gi);
+        mh[1] += a.corr[n + gi];
+        mh[2] += a.corr[2 * n + gi];
+        mh[3] += a.corr[3 * n + gi];
       }
     }
     if constexpr (CT) {
@@ -805,9 +805,9 @@ __global__ void __launch_bounds__(step_threads<TY>(), step_min_blocks<TY>()) mhd
   __shared__ unsigned long long tma_bar;
   __shared__ int tma_off;
   unsigned tma_phase = 0;
-  overlap_next();
   init_tma_barrier(&tma_bar, &tma_off);
   wait_previous();
+  overlap_next();
   long long q, qe;
   const int nzr = a.zhi - a.zlo;  // planes of this launch
   if (a.zparts > 0) {

@@ -7,6 +7,7 @@ import pytest
 
 import pmfmhd
 import problems
+from test_gpu_back_to_back import _form_bits, _form_state, _form_step
 
 pytestmark = pytest.mark.gpu
 DIMS = [(16, 16, 16), (33, 9, 40), (100, 75, 61), (40, 200, 7), (31, 8, 300)]
@@ -36,6 +37,24 @@ def test_division_of_the_work_leaves_the_bits(dims, solver):
         faces = [] if solver == "glm" else [s.ct.packed[:3 * s.nc].cpu().numpy()]
         out.append([pmfmhd.fields_to_host(s), pmfmhd.last_wavespeed(s), *faces])
         assert out[-1][1] == pytest.approx(pmfmhd.max_wavespeed(s), rel=1e-6)
+    for other in out[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(out[0], other))
+
+
+@pytest.mark.parametrize("dims", [(33, 9, 40), (100, 75, 61), (40, 200, 7), (224, 12, 224)])
+@pytest.mark.parametrize("form", ["comp", "ct_comp", "drag", "rad", "rad_ppm", "ct_rad"])
+def test_division_of_the_work_leaves_the_bits_of_every_form(dims, form):
+    """The forms that keep remainders or corrections; (224, 12, 224) is a box on which the radiation
+    step takes 13 rows of its own accord, more than the box has."""
+    out = []
+    for tile in (None, (8, dims[2]), (9, 1), (13, 3), (5, 16)):
+        s, corr = _form_state(form, dims)
+        if tile:
+            pmfmhd.set_tile(s, *tile)
+        dt, sp = pmfmhd.compute_dt(s, 0.2)
+        for _ in range(2):
+            _form_step(form, s, corr, dt, sp)
+        out.append(_form_bits(s, corr))
     for other in out[1:]:
         assert all(np.array_equal(a, b) for a, b in zip(out[0], other))
 
