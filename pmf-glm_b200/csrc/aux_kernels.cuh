@@ -70,8 +70,11 @@ inline dim3 col_grid(int nx, int ny, int nz, int sms, int* zc) {
 // memory traffic, so a cell is evaluated in FP64 only where an FP32 evaluation leaves it a chance
 // to exceed the maximum so far (of its warp, and of the blocks that had finished when this one
 // began): the FP32 sum of the six terms is off by less than eight roundings of the sum of their
-// magnitudes. The result is the FP64 maximum, bit for bit. The maximum is kept without the factor
-// 1/(2 dx) until the end (rounding is monotonic, so the factor commutes with it).
+// magnitudes and, where sums fall below the normal range, DIVB_TINY. A sum that left FP32's range
+// (inf, or NaN from inf - inf) is not below any bound, so its cell is evaluated. The result is the
+// FP64 maximum over the cells whose FP64 value is not a NaN, bit for bit. The maximum is kept without
+// the factor 1/(2 dx) until the end (rounding is monotonic, so the factor commutes with it).
+constexpr float DIVB_TINY = 1.5e-37f;  // twelve times the smallest normal number
 static __global__ void __launch_bounds__(AUX_THREADS) divb_kernel(const float* __restrict__ bx, const float* __restrict__ by,
                                                            const float* __restrict__ bz, int nx, int ny, int nz, int zc,
                                                            int bcx, int bcy, int bcz, double inv2dx,
@@ -89,7 +92,7 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb_kernel(const float* _
   const size_t top = bc_index(nz, nz, bcz, &fzp) * nxy;  // the plane above the last
   double m = 0.0;
   // a lower bound of the maximum (a millionth off, beyond the rounding of the division)
-  float lo = __double2float_rd(__longlong_as_double(*(volatile long long*)out_bits) / inv2dx * (1.0 - 1e-6));
+  float lo = __double2float_rd(__longlong_as_double(*(volatile long long*)out_bits) / inv2dx * (1.0 - 1e-6)) - DIVB_TINY;
   const size_t below = bc_index(z0 - 1, nz, bcz, &fzm) * nxy;
   float zm = bz[below + o] * fzm, z = bz[z0 * nxy + o];
   for (int k = z0; k < z1; ++k) {
@@ -99,11 +102,11 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb_kernel(const float* _
     const float xp = xr[oxp] * fxp, xm = xr[oxm] * fxm, yp = yr[oyp] * fyp, ym = yr[oym] * fym;
     const float d = (xp - xm) + (yp - ym) + (zp - zm);
     const float mag = fabsf(xp) + fabsf(xm) + fabsf(yp) + fabsf(ym) + fabsf(zp) + fabsf(zm);
-    const bool maybe = in && fmaf(4.7683716e-7f, mag, fabsf(d)) >= lo;  // 2^-21 mag
+    const bool maybe = in && !(fmaf(4.7683716e-7f, mag, fabsf(d)) < lo);  // 2^-21 mag
     if (maybe) {
       const double db = (double)xp - (double)xm + (double)yp - (double)ym + (double)zp - (double)zm;
       m = fmax(m, fabs(db));
-      lo = fmaxf(lo, __double2float_rd(m));
+      lo = fmaxf(lo, __double2float_rd(m) - DIVB_TINY);
     }
     if (__any_sync(0xffffffffu, maybe)) lo = warp_max(lo);
     zm = z;
@@ -132,7 +135,7 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb4_kernel(const float* 
   const size_t nxy = (size_t)nx * ny;
   const float* top = bz + bc_index(nz, nz, bcz, &fzp) * nxy + row + i;  // the plane above the last
   double m = 0.0;
-  float lo = __double2float_rd(__longlong_as_double(*(volatile long long*)out_bits) / inv2dx * (1.0 - 1e-6));
+  float lo = __double2float_rd(__longlong_as_double(*(volatile long long*)out_bits) / inv2dx * (1.0 - 1e-6)) - DIVB_TINY;
   auto ld4 = [](const float* p) { return *reinterpret_cast<const float4*>(p); };
   auto mul4 = [](float4 v, float f) { return make_float4(v.x * f, v.y * f, v.z * f, v.w * f); };
   const size_t below = bc_index(z0 - 1, nz, bcz, &fzm) * nxy;
@@ -146,19 +149,19 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb4_kernel(const float* 
     const float xp[4] = {c.y, c.z, c.w, xu}, xm[4] = {xl, c.x, c.y, c.z};
     const float ypa[4] = {yp.x, yp.y, yp.z, yp.w}, yma[4] = {ym.x, ym.y, ym.z, ym.w};
     const float zpa[4] = {zp.x, zp.y, zp.z, zp.w}, zma[4] = {zm.x, zm.y, zm.z, zm.w};
-    float reach = 0.0f;  // the largest the four may be
+    float reach = 0.0f;  // the largest the four may be (NaN if one of them is)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const float d = (xp[q] - xm[q]) + (ypa[q] - yma[q]) + (zpa[q] - zma[q]);
       const float mag = fabsf(xp[q]) + fabsf(xm[q]) + fabsf(ypa[q]) + fabsf(yma[q]) + fabsf(zpa[q]) + fabsf(zma[q]);
-      reach = fmaxf(reach, fmaf(4.7683716e-7f, mag, fabsf(d)));  // 2^-21 mag
+      reach = max_nan(reach, fmaf(4.7683716e-7f, mag, fabsf(d)));  // 2^-21 mag
     }
-    const bool maybe = in && reach >= lo;
+    const bool maybe = in && !(reach < lo);
     if (maybe) {
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         m = fmax(m, fabs((double)xp[q] - (double)xm[q] + (double)ypa[q] - (double)yma[q] + (double)zpa[q] - (double)zma[q]));
-      lo = fmaxf(lo, __double2float_rd(m));
+      lo = fmaxf(lo, __double2float_rd(m) - DIVB_TINY);
     }
     if (__any_sync(0xffffffffu, maybe)) lo = warp_max(lo);
     zm = z;

@@ -143,6 +143,12 @@ __device__ __forceinline__ float min_xorsign_abs(float a, float b) {
   asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
   return r;
 }
+// max(a, b), NaN if either is (fmaxf returns the other operand).
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 // Half the MonCen slope, 0.5*moncen(dl, dr) of glm_physics.jl:47-53, from dl, dr and
 // q = (dl+dr)/4. With the scalings by powers of two folded, the reference's value is
 // 0.5*sgn*min(2*min|dl|,|dr|, |(dl+dr)/2|) = sgn(q)*min(min(|dl|,|dr|), |q|) when dl*dr > 0 and
