@@ -56,14 +56,23 @@ static __global__ void __launch_bounds__(AUX_THREADS) wavespeed_kernel(const CPt
 
 // Column launches of the div-B kernels: one thread per (x, y) column of a 32 x 8 tile marches `zc`
 // planes, so that a cell's index costs no division and the z neighbours stay in registers. zc is
-// the longest chunk (of at most 16 planes) that still gives every SM eight blocks.
-constexpr int COL_X = 32, COL_Y = AUX_THREADS / 32;
-inline dim3 col_grid(int nx, int ny, int nz, int sms, int* zc) {
+// the longest chunk (of at most 16 planes) that still gives every SM eight blocks. Grid dimensions y
+// and z end at GRID_YZ: a taller box has its y tiles in grid dimension x (`yx`, the x tiles are then
+// few) and a deeper one longer chunks.
+constexpr int COL_X = 32, COL_Y = AUX_THREADS / 32, GRID_YZ = 65535;
+struct Cols {
+  int zc, yx;
+};
+inline dim3 col_grid(int nx, int ny, int nz, int sms, Cols* c) {
   const int tx = (nx + COL_X - 1) / COL_X, ty = (ny + COL_Y - 1) / COL_Y;
   const long long chunks = std::max(1LL, std::min((long long)nz, 8LL * sms / ((long long)tx * ty)));
-  *zc = (int)std::min(16LL, (nz + chunks - 1) / chunks);
-  return dim3(tx, ty, (nz + *zc - 1) / *zc);
+  c->zc = (int)std::max(std::min(16LL, (nz + chunks - 1) / chunks), ((long long)nz + GRID_YZ - 1) / GRID_YZ);
+  c->yx = ty > GRID_YZ;
+  const int tz = (nz + c->zc - 1) / c->zc;
+  return c->yx ? dim3(ty, tx, tz) : dim3(tx, ty, tz);
 }
+__device__ __forceinline__ int col_x(const Cols& c) { return (c.yx ? blockIdx.y : blockIdx.x) * COL_X + (threadIdx.x & 31); }
+__device__ __forceinline__ int col_y(const Cols& c) { return (c.yx ? blockIdx.x : blockIdx.y) * COL_Y + (threadIdx.x >> 5); }
 
 // max |div B| by BC-aware centred differences, in FP64 (diagnostics.jl:6-20).
 // In FP64 throughout, the conversions and adds of a cell cost several times its share of the
@@ -76,10 +85,10 @@ inline dim3 col_grid(int nx, int ny, int nz, int sms, int* zc) {
 // the factor 1/(2 dx) until the end (rounding is monotonic, so the factor commutes with it).
 constexpr float DIVB_TINY = 1.5e-37f;  // twelve times the smallest normal number
 static __global__ void __launch_bounds__(AUX_THREADS) divb_kernel(const float* __restrict__ bx, const float* __restrict__ by,
-                                                           const float* __restrict__ bz, int nx, int ny, int nz, int zc,
+                                                           const float* __restrict__ bz, int nx, int ny, int nz, Cols cols,
                                                            int bcx, int bcy, int bcz, double inv2dx,
                                                            unsigned long long* out_bits) {
-  const int ti = blockIdx.x * COL_X + (threadIdx.x & 31), tj = blockIdx.y * COL_Y + (threadIdx.x >> 5);
+  const int ti = col_x(cols), tj = col_y(cols);
   const bool in = ti < nx && tj < ny;
   const int i = min(ti, nx - 1), j = min(tj, ny - 1);
   float fxp, fxm, fyp, fym, fzm, fzp;
@@ -87,7 +96,7 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb_kernel(const float* _
   const unsigned oxp = row + bc_index(i + 1, nx, bcx, &fxp), oxm = row + bc_index(i - 1, nx, bcx, &fxm);
   const unsigned oyp = (unsigned)bc_index(j + 1, ny, bcy, &fyp) * nx + i;
   const unsigned oym = (unsigned)bc_index(j - 1, ny, bcy, &fym) * nx + i;
-  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
+  const int z0 = blockIdx.z * cols.zc, z1 = min(z0 + cols.zc, nz);
   const size_t nxy = (size_t)nx * ny;
   const size_t top = bc_index(nz, nz, bcz, &fzp) * nxy;  // the plane above the last
   double m = 0.0;
@@ -120,10 +129,10 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb_kernel(const float* _
 // scalar form executes 144 instructions a cell and warp, most of them for its indices, and takes
 // 119 us at 256^3, four times its traffic.
 static __global__ void __launch_bounds__(AUX_THREADS) divb4_kernel(const float* __restrict__ bx, const float* __restrict__ by,
-                                                            const float* __restrict__ bz, int nx, int ny, int nz, int zc,
+                                                            const float* __restrict__ bz, int nx, int ny, int nz, Cols cols,
                                                             int bcx, int bcy, int bcz, double inv2dx,
                                                             unsigned long long* out_bits) {
-  const int ti = (blockIdx.x * COL_X + (threadIdx.x & 31)) * 4, tj = blockIdx.y * COL_Y + (threadIdx.x >> 5);
+  const int ti = col_x(cols) * 4, tj = col_y(cols);
   const bool in = ti < nx && tj < ny;
   const int i = min(ti, nx - 4), j = min(tj, ny - 1);
   float fxp, fxm, fyp, fym, fzm, fzp;
@@ -131,7 +140,7 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb4_kernel(const float* 
   const unsigned oxp = row + bc_index(i + 4, nx, bcx, &fxp), oxm = row + bc_index(i - 1, nx, bcx, &fxm);
   const unsigned oyp = (unsigned)bc_index(j + 1, ny, bcy, &fyp) * nx + i;
   const unsigned oym = (unsigned)bc_index(j - 1, ny, bcy, &fym) * nx + i;
-  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
+  const int z0 = blockIdx.z * cols.zc, z1 = min(z0 + cols.zc, nz);
   const size_t nxy = (size_t)nx * ny;
   const float* top = bz + bc_index(nz, nz, bcz, &fzp) * nxy + row + i;  // the plane above the last
   double m = 0.0;
@@ -175,12 +184,12 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb4_kernel(const float* 
 static __global__ void __launch_bounds__(AUX_THREADS) divb_face_kernel(const float* __restrict__ bxf,
                                                                 const float* __restrict__ byf,
                                                                 const float* __restrict__ bzf, int nx, int ny,
-                                                                int nz, int zc, double invdx,
+                                                                int nz, Cols cols, double invdx,
                                                                 unsigned long long* out_bits) {
-  const int i = blockIdx.x * COL_X + (threadIdx.x & 31), j = blockIdx.y * COL_Y + (threadIdx.x >> 5);
+  const int i = col_x(cols), j = col_y(cols);
   double m = 0.0;
   if (i < nx && j < ny) {
-    const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
+    const int z0 = blockIdx.z * cols.zc, z1 = min(z0 + cols.zc, nz);
     const size_t nxy = (size_t)nx * ny, o = (size_t)j * nx + i;
     const size_t oip = (size_t)j * nx + wrap_inc(i, nx), ojp = (size_t)wrap_inc(j, ny) * nx + i;
     float z = bzf[z0 * nxy + o];

@@ -715,10 +715,10 @@ int pmfmhd_max_divb(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const U[9]
   // mostly empty
   bool v4 = g->nx % 4 == 0 && g->nx >= 64;
   for (int f = 5; f < 8; ++f) v4 = v4 && reinterpret_cast<uintptr_t>(U[f]) % 16 == 0;
-  int zc;
-  const dim3 tiles = col_grid(v4 ? g->nx / 4 : g->nx, g->ny, g->nz, c->sms, &zc);
+  Cols cols;
+  const dim3 tiles = col_grid(v4 ? g->nx / 4 : g->nx, g->ny, g->nz, c->sms, &cols);
   const auto kernel = v4 ? divb4_kernel : divb_kernel;
-  kernel<<<tiles, AUX_THREADS, 0, s>>>(U[5], U[6], U[7], g->nx, g->ny, g->nz, zc, g->bc[0], g->bc[1], g->bc[2],
+  kernel<<<tiles, AUX_THREADS, 0, s>>>(U[5], U[6], U[7], g->nx, g->ny, g->nz, cols, g->bc[0], g->bc[1], g->bc[2],
                                        1.0 / (2.0 * (double)g->dx), c->d_u64);
   PMF_CK(cudaGetLastError());
   PMF_CK(cudaMemcpyAsync(c->h_pin, c->d_u64, 8, cudaMemcpyDeviceToHost, s));
@@ -734,9 +734,9 @@ int pmfmhd_max_divb_face(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* ct, d
   cudaStream_t s = as_stream(stream);
   const long long nc = ncells(g);
   PMF_CK(cudaMemsetAsync(c->d_u64, 0, sizeof(unsigned long long), s));
-  int zc;
-  const dim3 tiles = col_grid(g->nx, g->ny, g->nz, c->sms, &zc);
-  divb_face_kernel<<<tiles, AUX_THREADS, 0, s>>>(ct, ct + nc, ct + 2 * nc, g->nx, g->ny, g->nz, zc,
+  Cols cols;
+  const dim3 tiles = col_grid(g->nx, g->ny, g->nz, c->sms, &cols);
+  divb_face_kernel<<<tiles, AUX_THREADS, 0, s>>>(ct, ct + nc, ct + 2 * nc, g->nx, g->ny, g->nz, cols,
                                                  1.0 / (double)g->dx, c->d_u64);
   PMF_CK(cudaGetLastError());
   PMF_CK(cudaMemcpyAsync(c->h_pin, c->d_u64, 8, cudaMemcpyDeviceToHost, s));
