@@ -387,20 +387,29 @@ __device__ __forceinline__ F9 hlld_x(const F9& L, const F9& R, float g, float bn
   const float x = degK ? 0.0f : (SM - uK) * (1.0f / denKK);
   const float ws = fmaf(fmaf(dSuK, x, 1.0f), fmaf(-bn * x, bt2, vbt), SMbn);
   const float sgn = copysignf(1.0f, bn);
-  const float t = outer ? 0.0f : SKs;
   const float y = outer ? SK * dKs * x : rK;
   const float cw = outer ? -SK * bn : sgn * SM * (denKK * (irK * iDK));
-  const float sqK = sgn * (left ? -sqL : sqR);
-  const float dt_ = dKs * t, by1 = fmaf(bn, y, bn), bu = fmaf(SSMK, y, uK);
+  const float by1 = fmaf(bn, y, bn), bu = fmaf(SSMK, y, uK);
   F9 f;
   f[0] = __fmul_rn(dKs, SM);
   f[1] = fmaf(f[0], SM, fmaf(-bn, bn, pts));
-  f[2] = fmaf(dt_, vyss - vK, fmaf(f[0], vK, -by1 * byK));
-  f[3] = fmaf(dt_, vzss - wK, fmaf(f[0], wK, -by1 * bzK));
-  f[4] = fmaf(iSSMK, fmaf(SM, fmaf(SK, pts, G), cw * ws), -sqK * t * wss);
+  f[2] = fmaf(f[0], vK, -by1 * byK);
+  f[3] = fmaf(f[0], wK, -by1 * bzK);
+  f[4] = __fmul_rn(iSSMK, fmaf(SM, fmaf(SK, pts, G), cw * ws));
   f[5] = fbn;
-  f[6] = fmaf(t, byss - byK, fmaf(bu, byK, -bn * vK));
-  f[7] = fmaf(t, bzss - bzK, fmaf(bu, bzK, -bn * wK));
+  f[6] = fmaf(bu, byK, -bn * vK);
+  f[7] = fmaf(bu, bzK, -bn * wK);
+  // The double-star terms enter in the inner region only, not as products with a zero: where the fast
+  // speed is below the rounding of u, S_M can equal the other side's S, whose single-star density and
+  // with it the double-star state is then not finite, while the flux of side K is.
+  if (!outer) {
+    const float t = SKs, m = dKs * t;
+    f[2] = fmaf(m, vyss - vK, f[2]);
+    f[3] = fmaf(m, vzss - wK, f[3]);
+    f[4] = fmaf(-sgn * (left ? -sqL : sqR) * t, wss, f[4]);
+    f[6] = fmaf(t, byss - byK, f[6]);
+    f[7] = fmaf(t, bzss - bzK, f[7]);
+  }
   f[8] = fpsi;
   return f;
 }

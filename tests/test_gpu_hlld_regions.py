@@ -43,3 +43,25 @@ def test_hlld_region_matches_oracle(region, dtol):
     for v in range(9):
         lim = PAR["atol"] + PAR["rtol"] * np.abs(o64.U[v]).max() + np.abs(o32.U[v] - o64.U[v]).max()
         assert np.abs(host[v] - o64.U[v]).max() <= lim, (region, v)
+
+
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_hypersonic_drift_stays_finite(sign):
+    """A drift whose fast speed (pressure at its floor) is below the rounding of the velocity: the
+    contact speed then equals the far side's signal speed to the last bit."""
+    dims = (34, 11, 9)
+    i, j, k = problems.cell_coords(dims)
+    x, y, z = (2 * np.pi * (a - 0.5) / n for a, n in zip((i, j, k), dims))
+    rho = 1 + 1e-3 * np.sin(x + y)
+    v = [sign * 2e4 * (1 + 1e-6 * np.sin(z)), sign * 3e4 * (1 + 1e-4 * np.sin(y)), -sign * 1e4 + 0 * x]
+    B = [1e-4 * np.sin(y - z), 1e-4 * np.sin(z + x), 1e-4 * np.sin(x + y)]
+    E = 0.5 * rho * sum(a * a for a in v) * (1 - 1e-6)
+    U = np.array([rho, *(rho * a for a in v), E, *B, 0 * x]).astype(np.float32)
+    o = oracle.OracleState(dims, 1.0 / 34, hlld_dtol_rel=1e-5, dtype=np.float32)
+    dev = pmfmhd.set_fields(pmfmhd.allocate_state(dims, 1.0 / 34), U)
+    o.U[:] = U
+    dt, sp = o.compute_dt(0.2)
+    for _ in range(2):
+        o.step(dt, ch=sp)
+        pmfmhd.step(dev, float(dt), ch=float(sp))
+    assert np.isfinite(o.U).all() and np.isfinite(pmfmhd.fields_to_host(dev)).all()
