@@ -143,6 +143,12 @@ __device__ __forceinline__ float min_xorsign_abs(float a, float b) {
   asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
   return r;
 }
+// The same, NaN if either is (the form above returns the other operand's magnitude).
+__device__ __forceinline__ float min_xorsign_abs_nan(float a, float b) {
+  float r;
+  asm("min.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 // max(a, b), NaN if either is (fmaxf returns the other operand).
 __device__ __forceinline__ float max_nan(float a, float b) {
   float r;
@@ -167,13 +173,13 @@ __device__ __forceinline__ float half_moncen(float dl, float dr, float q) {
 // zero where their signs agree: z = max(-min.xorsign(L, R), 0) is that smaller magnitude or
 // zero. No branch and no division (the reference's form diverges within a warp and divides
 // twice a field: the 192^3 PPM/HLLD step took 1.39 ms with it, 0.73 with this form and the
-// solver above).
+// solver below). A NaN difference gives NaN offsets, as the reference's form does.
 __device__ __forceinline__ void ppm_offsets(float dl, float dr, float& oL, float& oR) {
   const float s = 0.25f * (dl + dr), c = dr - dl;
   const float L = fmaf(1.0f / 12.0f, c, -s), R = fmaf(1.0f / 12.0f, c, s);
-  const float z2 = 2.0f * fmaxf(-min_xorsign_abs(L, R), 0.0f);
-  oL = min_xorsign_abs(L, z2);
-  oR = min_xorsign_abs(R, z2);
+  const float z2 = 2.0f * max_nan(-min_xorsign_abs_nan(L, R), 0.0f);
+  oL = min_xorsign_abs_nan(L, z2);
+  oR = min_xorsign_abs_nan(R, z2);
 }
 
 template <int RECON>

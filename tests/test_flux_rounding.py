@@ -87,3 +87,36 @@ def test_rounding_error_is_not_above_the_reference_form(host, mach, beta, jump):
     for c in (0, 1, 2, 3, 4, 6, 7):
         e_dev, e_ref = (np.sqrt(((f[:, c] - ref[:, c]) ** 2).mean()) for f in (dev, f32))
         assert e_dev <= 1.1 * e_ref, (c, e_dev / e_ref)
+
+
+def _ppm(host, dl, dr):
+    dl, dr = (np.ascontiguousarray(a, np.float32) for a in (dl, dr))
+    oL, oR = np.zeros_like(dl), np.zeros_like(dl)
+    host.ppm(len(dl), _ptr(dl), _ptr(dr), _ptr(oL), _ptr(oR))
+    return oL, oR
+
+
+def test_ppm_offsets_pass_on_what_is_not_finite(host):
+    bad = [np.nan, np.inf, -np.inf]
+    pairs = np.array([(a, b) for a in bad + [0.5, -0.5, 0.0] for b in bad + [0.5, -0.5, 0.0]])
+    pairs = pairs[~np.isfinite(pairs).all(1)]
+    oL, oR = _ppm(host, pairs[:, 0], pairs[:, 1])
+    nan = np.isnan(pairs).any(1)
+    assert np.isnan(oL[nan]).all() and np.isnan(oR[nan]).all()
+    assert not np.isfinite(oL).any() and not np.isfinite(oR).any()
+
+
+def test_ppm_offsets_are_the_reference_cases(host):
+    rng = np.random.default_rng(2)
+    dl, dr = (rng.standard_normal(100000).astype(np.float32) for _ in range(2))
+    dl[:1000], dr[500:1500] = 0, 0
+    oL, oR = _ppm(host, dl, dr)
+    s, c = (dl.astype(np.float64) + dr) / 4, (dr.astype(np.float64) - dl) / 12
+    L, R = c - s, c + s  # edges less the mean (glm_physics.jl:188-200)
+    d, mid = R - L, 0.5 * (L + R)
+    diff, lim = -mid * d, d * d / 6
+    eL = np.where(-R * L <= 0, 0, np.where(diff > lim, -2 * R, L))
+    eR = np.where(-R * L <= 0, 0, np.where(diff > lim, R, np.where(diff < -lim, -2 * L, R)))
+    # three roundings of terms below |dl| + |dr|; at a tie of two cases their values agree
+    tol = 4 * 2.0 ** -24 * (np.abs(dl) + np.abs(dr))
+    assert np.all(np.abs(oL - eL) <= tol) and np.all(np.abs(oR - eR) <= tol)
