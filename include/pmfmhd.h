@@ -357,8 +357,7 @@ int pmfmhd_terminal_velocity_max(pmfmhd_ctx* ctx, const pmfmhd_grid* g, const fl
  * NULL) or edge-averaged face curl (CT, faces Kahan-compensated through the packed
  * remainders when `compensate`), order-2 or order-4 dissipation with eta from vmax; E
  * follows the magnetic energy. Density and thermal energy are held. scratch (9 arrays) and
- * the CT workspace slots are overwritten. (The CT cell-EMF slots are also written when the call
- * is refused for its subcycle limit.) Outputs nsub, vmax, eta (nullable).
+ * the CT workspace slots are overwritten; a refused call writes neither. Outputs nsub, vmax, eta (nullable).
  */
 int pmfmhd_terminal_ct_induction(pmfmhd_ctx* ctx, const pmfmhd_grid* g, float* const U[9], float* const scratch[9],
                                  float* ct_packed, float dt, float gamma_drag, float pressure_coeff, float cfl,

@@ -445,14 +445,14 @@ int cube_of(const pmfmhd_grid* g, Cube* G) {
 namespace pmf {
 namespace {
 using namespace host;
-// Maximum terminal speed of U (blocking); with ec also the cell EMF of the same field, from the same
-// pass.
+// Maximum terminal speed of U (blocking). Nothing of the caller's is written: the call that asks may
+// still be refused for its subcycle limit. (Keeping the EMF of this pass for the first stage would
+// save a 128^3 CT subcycle one of its six passes.)
 int velocity_max(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const* U, Cube G, const dim3& tiles,
-                 const Terminal& P, float* const* ec, double* vmax, cudaStream_t s) {
+                 const Terminal& P, double* vmax, cudaStream_t s) {
   PMF_CK(cudaMemsetAsync(c->d_u64, 0, sizeof(unsigned int), s));
   unsigned int* bits = reinterpret_cast<unsigned int*>(c->d_u64);
-  cell_emf_kernel<<<tiles, kT, 0, s>>>(U[0], Field3{U[5], U[6], U[7]}, ec ? ec[0] : nullptr, ec ? ec[1] : nullptr,
-                                       ec ? ec[2] : nullptr, bits, G, P);
+  cell_emf_kernel<<<tiles, kT, 0, s>>>(U[0], Field3{U[5], U[6], U[7]}, nullptr, nullptr, nullptr, bits, G, P);
   PMF_CK(cudaGetLastError());
   PMF_CK(cudaMemcpyAsync(c->h_pin, bits, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
   PMF_CK(cudaStreamSynchronize(s));
@@ -495,7 +495,7 @@ int pmfmhd_terminal_velocity_max(pmfmhd_ctx* c, const pmfmhd_grid* g, const floa
   if ((rc = cube_of(g, &G))) return rc;
   const dim3 tiles = tiles_of(G, c->sms);
   const Terminal P{1.0f / (2.0f * g->dx), gamma_drag, pressure_coeff, g->smallr, vcap};
-  return velocity_max(c, g, U, G, tiles, P, nullptr, vmax, reinterpret_cast<cudaStream_t>(stream));
+  return velocity_max(c, g, U, G, tiles, P, vmax, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int pmfmhd_terminal_ct_induction(pmfmhd_ctx* c, const pmfmhd_grid* g, float* const U[9], float* const scratch[9],
@@ -517,13 +517,8 @@ int pmfmhd_terminal_ct_induction(pmfmhd_ctx* c, const pmfmhd_grid* g, float* con
   const dim3 tiles = tiles_of(G, c->sms);
   const Terminal P{1.0f / (2.0f * g->dx), gamma_drag, pressure_coeff, g->smallr, vcap};
   auto slot = [&](int q) { return ct + (size_t)q * n; };
-  // CT: the cell EMF of the first stage lands in its workspace slots in the same pass (the GLM form
-  // keeps it in the caller's scratch fields, which a refused call leaves alone)
-  float* ecs[3] = {};
-  if (ct != nullptr)
-    for (int d = 0; d < 3; ++d) ecs[d] = slot(CT_ECX + d);
   double vmax = 0.0;
-  if ((rc = velocity_max(c, g, U, G, tiles, P, ct != nullptr ? ecs : nullptr, &vmax, s))) return rc;
+  if ((rc = velocity_max(c, g, U, G, tiles, P, &vmax, s))) return rc;
   const double dx = (double)g->dx;
   const long long nsub = std::max<long long>(
       1, (long long)std::ceil((double)dt * vmax / std::max((double)cfl * dx, DBL_EPSILON)));
@@ -554,8 +549,7 @@ int pmfmhd_terminal_ct_induction(pmfmhd_ctx* c, const pmfmhd_grid* g, float* con
       const Field3 ec{slot(CT_ECX), slot(CT_ECY), slot(CT_ECZ)};
       const auto stage0 = o4 ? face_stage_kernel<4, 0> : face_stage_kernel<2, 0>;
       const auto stage1 = o4 ? face_stage_kernel<4, 1> : face_stage_kernel<2, 1>;
-      if (it > 0)
-        cell_emf_kernel<<<tiles, kT, 0, s>>>(U[0], B, slot(CT_ECX), slot(CT_ECY), slot(CT_ECZ), nullptr, G, P);
+      cell_emf_kernel<<<tiles, kT, 0, s>>>(U[0], B, slot(CT_ECX), slot(CT_ECY), slot(CT_ECZ), nullptr, G, P);
       stage0<<<tiles, kT, 0, s>>>(ec, slot(CT_BXF), slot(CT_BYF), slot(CT_BZF), slot(CT_MFX), slot(CT_MFY),
                                   slot(CT_MFZ), nullptr, nullptr, nullptr, G, S, 0);
       face_average_kernel<<<tiles, kT, 0, s>>>(slot(CT_MFX), slot(CT_MFY), slot(CT_MFZ), scratch[5], scratch[6],
