@@ -10,6 +10,7 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "../../include/pmfmhd.h"
@@ -115,26 +116,38 @@ Split split_work(long long cols, int nz, long long slots, int tz) {
   return s;
 }
 
-// Tile height of an untuned grid: the height whose longest CTA takes least, its planes times the
-// relative time of one plane of a full GPU. Measured at 256^3: 3.4, 3.85 us a plane at 8 and 9
-// rows for GLM, 3.5, 4.15 for CT, 5.1, 5.6, 7.6 at 8, 9 and 13 for the radiation-coupled step
-// (which waits on its loads of the correction arrays, so that its 16 warps at 13 rows pay; the
-// others are slower at 13 rows for every size). A grid under 8 rows takes the 5-row tile.
+// Time of one plane of the longest CTA at 9 and 13 rows, relative to 8 rows, measured on full GPUs
+// (128^3, 256^3: us per step over Split::longest; CT without its companion kernels).
+//   9 rows: 1.08-1.13 for GLM (plain, compensated, drag-coupled), 1.15-1.18 for CT, 1.10 radiation-coupled.
+//   13 rows: 1.67-1.80 for GLM and CT. The radiation-coupled step waits on its loads of the correction
+//   arrays, so that its 16 warps at 13 rows pay more often: 1.52 for PLM with HLLD, 1.55 with minmod, 1.58
+//   with HLL or LLF; but its PPM and CT instantiations spill there: 1.66 for PPM, 1.64-1.72 for CT with
+//   PLM, 1.9 for CT with PPM (1.7 in chunks of a few planes).
+struct RowCost {
+  double nine, thirteen;
+};
+RowCost row_cost(const pmfmhd_grid* g, bool ct, int src) {
+  if (src != SRC_RAD) return ct ? RowCost{1.18, 1.80} : RowCost{1.13, 1.80};
+  const bool ppm = g->recon == PMFMHD_RECON_PPM, hlld = g->riemann == PMFMHD_RIEMANN_HLLD;
+  return RowCost{1.10, ct ? (ppm ? 1.80 : 1.65) : ppm ? 1.66 : hlld ? 1.52 : 1.58};
+}
+
+// Tile height of an untuned grid: the height whose longest CTA takes least. A grid under 8 rows takes
+// the 5-row tile. (With the PLM/HLLD radiation step's ratio for every form, and 13 rows closed to the
+// others, the 128^3 radiation step took 356 against 321 us with PPM, 433 against 354 in CT with PPM, and
+// a 224x12x224 GLM step 89 against 75.)
 Tune default_tune(const pmfmhd_ctx* c, const pmfmhd_grid* g, bool ct, int src) {
   if (g->ny < 8) return Tune{5, 1};
-  struct Cost {
-    int ty;
-    double glm, ct, rad;
-  };
-  constexpr Cost kCost[] = {{8, 1.0, 1.0, 1.0}, {9, 1.13, 1.18, 1.10}, {13, 1e9, 1e9, 1.50}};
+  const RowCost rc = row_cost(g, ct, src);
+  const std::pair<int, double> heights[] = {{8, 1.0}, {9, rc.nine}, {13, rc.thirteen}};
   Tune best{8, 1};
   double least = 1e300;
-  for (const Cost& k : kCost) {
-    const long long cols = (long long)((g->nx + TILE_X - 1) / TILE_X) * ((g->ny + k.ty - 1) / k.ty);
-    const double cost = (double)split_work(cols, g->nz, c->sms, 1).longest * (src == SRC_RAD ? k.rad : ct ? k.ct : k.glm);
+  for (const auto& [ty, plane] : heights) {
+    const long long cols = (long long)((g->nx + TILE_X - 1) / TILE_X) * ((g->ny + ty - 1) / ty);
+    const double cost = (double)split_work(cols, g->nz, c->sms, 1).longest * plane;
     if (cost < least) {
       least = cost;
-      best.ty = k.ty;
+      best.ty = ty;
     }
   }
   return best;
@@ -220,11 +233,13 @@ int occupancy_of(const StepKernelInfo& k) {
   return occ;
 }
 
-// Whether a box's launches overlap the previous kernel of the stream (overlap_next / wait_previous in
-// the kernels): the launch latency, some 2 us a kernel, is then hidden behind that kernel's tail
-// (32^3 GLM step 16.4 -> 14.1 us, 48^3 CT 39.8 -> 32.4, 128^3 CT 275 -> 270). Past about 160^3 cells
-// it is nothing beside the kernels, whose last CTAs the early CTAs then disturb (256^3 CT 1.957
-// -> 1.967 ms).
+// Whether a box's launches overlap the previous kernel of the stream (wait_previous / overlap_next in
+// the kernels): the launch latency, some 2 us a kernel, is then hidden behind that kernel's tail.
+// Launched back to back in a stream, with and without: GLM 14.3 / 16.4 us at 32^3, 38.4 / 39.5 at 64^3,
+// 93.4 / 94.2 at 96^3, 322 / 326 at 144^3; CT 32.7 / 39.6 at 48^3, 119 / 127 at 96^3, 506 / 511 at 160^3;
+// radiation 16.3 / 17.3 at 32^3, 435 / 439 at 144^3 (but 49.8 / 47.2 at 64^3). From 176^3 on nothing is
+// gained and from 224^3 half a percent lost (GLM 1036 / 1033), as it is in graphs from 128^3 on. The
+// line lies at 161^3.
 bool overlaps(const pmfmhd_grid* g) { return ncells(g) <= (1LL << 22); }
 
 cudaError_t launch_kernel(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t s,
