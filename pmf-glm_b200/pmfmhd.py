@@ -185,8 +185,8 @@ def _stream():
 
 
 def _p9(ts) -> "ctypes.Array":
-    a = _P9()
-    a[:] = [t.data_ptr() for t in ts]  # a third of the time of passing nine arguments
+    a, p = _P9(), [t.data_ptr() for t in ts]
+    a[:len(p)] = p  # a third of the time of passing nine arguments; missing fields are null pointers
     return a
 
 
