@@ -55,24 +55,19 @@ struct Column {
   unsigned x[5], y[5];  // x[2 + d], y[2 + d]: wrapped x index and row offset at distance d
   int z0, z1;
   bool in;
-  __device__ __forceinline__ static int wrap(int i, int n) {
-    while (i < 0) i += n;
-    while (i >= n) i -= n;
-    return i;
-  }
   __device__ __forceinline__ explicit Column(const Cube& G) : N(G.N), nxy(G.N * G.N) {
     const int i = blockIdx.x * kX + (threadIdx.x & (kX - 1)), j = blockIdx.y * kY + threadIdx.x / kX;
     in = i < N && j < N;
 #pragma unroll
     for (int d = -2; d <= 2; ++d) {
-      x[2 + d] = wrap(i + d, N);
-      y[2 + d] = wrap(j + d, N) * N;
+      x[2 + d] = wrap_index(i + d, N);
+      y[2 + d] = wrap_index(j + d, N) * N;
     }
     z0 = blockIdx.z * G.zc;
     z1 = min(z0 + G.zc, N);
   }
   __device__ __forceinline__ unsigned at(int dx, int dy) const { return y[2 + dy] + x[2 + dx]; }
-  __device__ __forceinline__ unsigned plane(int k) const { return (unsigned)(wrap(k, N) * nxy); }
+  __device__ __forceinline__ unsigned plane(int k) const { return (unsigned)(wrap_index(k, N) * nxy); }
 };
 
 struct F3 {
@@ -253,7 +248,6 @@ template <int ORDER> struct Dissip {
 
 struct Stage {
   float dt, inv2dx, invdx, invdx2, eta;
-  int order;
 };
 
 // GLM SSPRK2 stage (terminal_ct.jl:240-293). STAGE 0: out = B + dt*rhs(e, B).
@@ -530,7 +524,6 @@ int pmfmhd_terminal_ct_induction(pmfmhd_ctx* c, const pmfmhd_grid* g, float* con
   S.invdx2 = 1.0f / (g->dx * g->dx);
   S.eta = dissipation_order == 4 ? (float)(dissipation / 12.0) * (float)vmax * (g->dx * g->dx * g->dx)
                                  : dissipation * (float)vmax * g->dx;
-  S.order = dissipation_order;
   const bool o4 = dissipation_order == 4;
   const Field3 B{U[5], U[6], U[7]}, Bp{scratch[5], scratch[6], scratch[7]};  // the predictor's cell B
   for (long long it = 0; it < nsub; ++it) {
