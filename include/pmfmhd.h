@@ -58,8 +58,8 @@ typedef struct pmfmhd_grid {
   float dx, gamma, smallr, pfl, llf_dmin, llf_pmin;
   /* HLLD single-star states (glm_physics.jl:255-263) fall back to the unmodified transverse
    * state when |denK| < max(1e-12, hlld_dtol_rel * bn^2), denK = d(S-u)(S-SM) - bn^2.
-   * 0 (PMFMHD_HLLD_DTOL_REFERENCE) is the reference's own absolute test |denK| < 1e-12: the
-   * reference's arithmetic exactly. 1e-5 (PMFMHD_HLLD_DTOL_RELATIVE) widens it to the FP32
+   * 0 (PMFMHD_HLLD_DTOL_REFERENCE) is the reference's own absolute test |denK| < 1e-12 (the flux
+   * around it is rearranged either way). 1e-5 (PMFMHD_HLLD_DTOL_RELATIVE) widens it to the FP32
    * rounding level of denK, where the single-star states are otherwise ~1/denK of rounding
    * noise; it changes the flux only at those near-degenerate faces (a handful per step on a
    * turbulent 256^3 box) and kept a 512^3 turbulent box finite that blew up with the absolute

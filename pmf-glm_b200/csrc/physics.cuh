@@ -330,8 +330,9 @@ __device__ __forceinline__ F9 hll_x(const F9& L, const F9& R, float g, float bn,
 // where a face holds a head-on collision of more than Mach 10 (normal momentum, 1.1) or an
 // expansion of that strength (induction, 1.1-1.7; the other components 0.02-0.6).
 // The step is bounded by instruction issue: with this form, the predictor's sums in multiply-adds
-// and the vectorised tile edges the 256^3 GLM step executes 58 instead of 72 warp instructions
-// per cell (1.77 -> 1.54 ms; constrained transport 2.29 -> 2.05 ms).
+// and the vectorised tile edges the 256^3 GLM step executes 59.7 instead of 71.8 warp
+// instructions per cell (1.77 -> 1.55 ms, 1 % of it spent on the side's own flux; constrained
+// transport 2.29 -> 2.05 ms).
 __device__ __forceinline__ F9 hlld_x(const F9& L, const F9& R, float g, float bn, float fbn, float fpsi,
                                      float dtol_rel, HlldCensus* cen = nullptr) {
   const float2 d = p2(L[0], R[0]), u = p2(L[1], R[1]), v = p2(L[2], R[2]), w = p2(L[3], R[3]);
