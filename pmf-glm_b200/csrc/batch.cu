@@ -381,7 +381,7 @@ int pmfmhd_batch_step(pmfmhd_batch* b, int nsteps, void* stream) {
   for (int n = 0; n < nsteps; ++n) {
     const int p = b->parity;
     if (b->graph[p] == nullptr) {
-      std::lock_guard<std::mutex> lk(c->mu);
+      std::lock_guard<std::mutex> lk(c->cap_mu);
       PMF_CK(cudaStreamBeginCapture(c->cap, cudaStreamCaptureModeThreadLocal));
       int rc = enqueue_batch_step(b, p, c->cap);
       cudaGraph_t graph = nullptr;

@@ -842,7 +842,7 @@ int pmfmhd_run_glm(pmfmhd_ctx* c, const pmfmhd_grid* g, float* const U[9], float
   std::memcpy(k, &t.ty, 4); k += 4;
   std::memcpy(k, &t.tz, 4); k += 4;
   cudaStream_t s = as_stream(stream);
-  std::lock_guard<std::mutex> lk(c->mu);
+  std::lock_guard<std::mutex> lk(c->cap_mu);
   for (auto& e : c->graphs) {
     if (e.key == key) {
       PMF_CK(cudaGraphLaunch(e.exec, s));

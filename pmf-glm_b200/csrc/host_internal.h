@@ -92,7 +92,8 @@ struct pmfmhd_ctx {
   int tma_stall_polls = 0;                         // pmfmhd_set_tma_stall test hook
   float* d_mask = nullptr;                         // copy of a radiation fallback mask (masked step
   long long mask_cells = 0;                        // with density tracking), allocated on first use
-  std::mutex mu;
+  std::mutex mu;      // tune, maps, d_mask
+  std::mutex cap_mu;  // cap while it records, graphs; the recorded launches take `mu` themselves
 };
 
 namespace pmf {
