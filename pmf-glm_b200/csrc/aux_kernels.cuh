@@ -56,23 +56,20 @@ static __global__ void __launch_bounds__(AUX_THREADS) wavespeed_kernel(const CPt
 
 // Column launches of the div-B kernels: one thread per (x, y) column of a 32 x 8 tile marches `zc`
 // planes, so that a cell's index costs no division and the z neighbours stay in registers. zc is
-// the longest chunk (of at most 16 planes) that still gives every SM eight blocks. Grid dimensions y
-// and z end at GRID_YZ: a taller box has its y tiles in grid dimension x (`yx`, the x tiles are then
-// few) and a deeper one longer chunks.
-constexpr int COL_X = 32, COL_Y = AUX_THREADS / 32, GRID_YZ = 65535;
-struct Cols {
-  int zc, yx;
-};
-inline dim3 col_grid(int nx, int ny, int nz, int sms, Cols* c) {
+// the longest chunk (of at most 16 planes) that still gives every SM eight blocks.
+constexpr int COL_X = 32, COL_Y = AUX_THREADS / 32, COL_Z = 16;
+inline dim3 col_grid(int nx, int ny, int nz, int sms, int* zc) {
   const int tx = (nx + COL_X - 1) / COL_X, ty = (ny + COL_Y - 1) / COL_Y;
   const long long chunks = std::max(1LL, std::min((long long)nz, 8LL * sms / ((long long)tx * ty)));
-  c->zc = (int)std::max(std::min(16LL, (nz + chunks - 1) / chunks), ((long long)nz + GRID_YZ - 1) / GRID_YZ);
-  c->yx = ty > GRID_YZ;
-  const int tz = (nz + c->zc - 1) / c->zc;
-  return c->yx ? dim3(ty, tx, tz) : dim3(tx, ty, tz);
+  *zc = (int)std::min((long long)COL_Z, (nz + chunks - 1) / chunks);
+  return dim3(tx, ty, (nz + *zc - 1) / *zc);
 }
-__device__ __forceinline__ int col_x(const Cols& c) { return (c.yx ? blockIdx.y : blockIdx.x) * COL_X + (threadIdx.x & 31); }
-__device__ __forceinline__ int col_y(const Cols& c) { return (c.yx ? blockIdx.x : blockIdx.y) * COL_Y + (threadIdx.x >> 5); }
+// Where columns pay: tiles at least half full (a 1 x 600 x 600 box took 67 us by columns and takes 31
+// with one thread per cell, 8 x 512 x 512 55 and 43), within what grid dimensions y and z can count.
+inline bool cols_pay(int nx, int ny, int nz) {
+  const long long tx = (nx + COL_X - 1) / COL_X, ty = (ny + COL_Y - 1) / COL_Y;
+  return 2LL * nx * ny >= tx * ty * AUX_THREADS && ty <= 65535 && nz <= 65535LL * COL_Z;
+}
 
 // max |div B| by BC-aware centred differences, in FP64 (diagnostics.jl:6-20).
 // In FP64 throughout, the conversions and adds of a cell cost several times its share of the
@@ -85,10 +82,10 @@ __device__ __forceinline__ int col_y(const Cols& c) { return (c.yx ? blockIdx.x 
 // the factor 1/(2 dx) until the end (rounding is monotonic, so the factor commutes with it).
 constexpr float DIVB_TINY = 1.5e-37f;  // twelve times the smallest normal number
 static __global__ void __launch_bounds__(AUX_THREADS) divb_kernel(const float* __restrict__ bx, const float* __restrict__ by,
-                                                           const float* __restrict__ bz, int nx, int ny, int nz, Cols cols,
-                                                           int bcx, int bcy, int bcz, double inv2dx,
+                                                           const float* __restrict__ bz, int nx, int ny, int nz, int zc,
+                                                           int bcx, int bcy, int bcz, double inv2dx, double twodx,
                                                            unsigned long long* out_bits) {
-  const int ti = col_x(cols), tj = col_y(cols);
+  const int ti = blockIdx.x * COL_X + (threadIdx.x & 31), tj = blockIdx.y * COL_Y + (threadIdx.x >> 5);
   const bool in = ti < nx && tj < ny;
   const int i = min(ti, nx - 1), j = min(tj, ny - 1);
   float fxp, fxm, fyp, fym, fzm, fzp;
@@ -96,12 +93,12 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb_kernel(const float* _
   const unsigned oxp = row + bc_index(i + 1, nx, bcx, &fxp), oxm = row + bc_index(i - 1, nx, bcx, &fxm);
   const unsigned oyp = (unsigned)bc_index(j + 1, ny, bcy, &fyp) * nx + i;
   const unsigned oym = (unsigned)bc_index(j - 1, ny, bcy, &fym) * nx + i;
-  const int z0 = blockIdx.z * cols.zc, z1 = min(z0 + cols.zc, nz);
+  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
   const size_t nxy = (size_t)nx * ny;
   const size_t top = bc_index(nz, nz, bcz, &fzp) * nxy;  // the plane above the last
   double m = 0.0;
-  // a lower bound of the maximum (a millionth off, beyond the rounding of the division)
-  float lo = __double2float_rd(__longlong_as_double(*(volatile long long*)out_bits) / inv2dx * (1.0 - 1e-6)) - DIVB_TINY;
+  // a lower bound of the maximum (twodx: a millionth below 1 / inv2dx, beyond its rounding)
+  float lo = __double2float_rd(__longlong_as_double(*(volatile long long*)out_bits) * twodx) - DIVB_TINY;
   const size_t below = bc_index(z0 - 1, nz, bcz, &fzm) * nxy;
   float zm = bz[below + o] * fzm, z = bz[z0 * nxy + o];
   for (int k = z0; k < z1; ++k) {
@@ -129,10 +126,10 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb_kernel(const float* _
 // scalar form executes 144 instructions a cell and warp, most of them for its indices, and takes
 // 119 us at 256^3, four times its traffic.
 static __global__ void __launch_bounds__(AUX_THREADS) divb4_kernel(const float* __restrict__ bx, const float* __restrict__ by,
-                                                            const float* __restrict__ bz, int nx, int ny, int nz, Cols cols,
-                                                            int bcx, int bcy, int bcz, double inv2dx,
+                                                            const float* __restrict__ bz, int nx, int ny, int nz, int zc,
+                                                            int bcx, int bcy, int bcz, double inv2dx, double twodx,
                                                             unsigned long long* out_bits) {
-  const int ti = col_x(cols) * 4, tj = col_y(cols);
+  const int ti = (blockIdx.x * COL_X + (threadIdx.x & 31)) * 4, tj = blockIdx.y * COL_Y + (threadIdx.x >> 5);
   const bool in = ti < nx && tj < ny;
   const int i = min(ti, nx - 4), j = min(tj, ny - 1);
   float fxp, fxm, fyp, fym, fzm, fzp;
@@ -140,11 +137,11 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb4_kernel(const float* 
   const unsigned oxp = row + bc_index(i + 4, nx, bcx, &fxp), oxm = row + bc_index(i - 1, nx, bcx, &fxm);
   const unsigned oyp = (unsigned)bc_index(j + 1, ny, bcy, &fyp) * nx + i;
   const unsigned oym = (unsigned)bc_index(j - 1, ny, bcy, &fym) * nx + i;
-  const int z0 = blockIdx.z * cols.zc, z1 = min(z0 + cols.zc, nz);
+  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
   const size_t nxy = (size_t)nx * ny;
   const float* top = bz + bc_index(nz, nz, bcz, &fzp) * nxy + row + i;  // the plane above the last
   double m = 0.0;
-  float lo = __double2float_rd(__longlong_as_double(*(volatile long long*)out_bits) / inv2dx * (1.0 - 1e-6)) - DIVB_TINY;
+  float lo = __double2float_rd(__longlong_as_double(*(volatile long long*)out_bits) * twodx) - DIVB_TINY;
   auto ld4 = [](const float* p) { return *reinterpret_cast<const float4*>(p); };
   auto mul4 = [](float4 v, float f) { return make_float4(v.x * f, v.y * f, v.z * f, v.w * f); };
   const size_t below = bc_index(z0 - 1, nz, bcz, &fzm) * nxy;
@@ -180,16 +177,49 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb4_kernel(const float* 
   if (threadIdx.x == 0) atomicMax(out_bits, (unsigned long long)__double_as_longlong(m * inv2dx));
 }
 
+// One thread per cell in turn, for boxes whose columns would leave most lanes idle.
+static __global__ void __launch_bounds__(AUX_THREADS) divb_flat_kernel(const float* __restrict__ bx,
+                                                                const float* __restrict__ by,
+                                                                const float* __restrict__ bz, int nx, int ny,
+                                                                int nz, int bcx, int bcy, int bcz, double inv2dx,
+                                                                unsigned long long* out_bits) {
+  const unsigned nc = (unsigned)nx * ny * nz, step = gridDim.x * blockDim.x;  // nc < 2^31, step < 2^20
+  // images of the two indices just outside each axis, and the wall's sign there
+  int hi[3], lo[3];
+  float fh[3], fl[3];
+  const int n[3] = {nx, ny, nz}, code[3] = {bcx, bcy, bcz};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    hi[a] = bc_index(n[a], n[a], code[a], &fh[a]);
+    lo[a] = bc_index(-1, n[a], code[a], &fl[a]);
+  }
+  double m = 0.0;
+  for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += step) {
+    const int q = c / (unsigned)nx, i = c - q * nx, k = q / ny, j = q - k * ny;
+    auto at = [&](int a, int b, int d) { return (d * ny + b) * nx + a; };
+    auto up = [&](int x, int a) { return x + 1 < n[a] ? x + 1 : hi[a]; };
+    auto down = [&](int x, int a) { return x > 0 ? x - 1 : lo[a]; };
+    auto su = [&](int x, int a) { return x + 1 < n[a] ? 1.0f : fh[a]; };
+    auto sd = [&](int x, int a) { return x > 0 ? 1.0f : fl[a]; };
+    const double db = (double)(bx[at(up(i, 0), j, k)] * su(i, 0)) - (double)(bx[at(down(i, 0), j, k)] * sd(i, 0)) +
+                      (double)(by[at(i, up(j, 1), k)] * su(j, 1)) - (double)(by[at(i, down(j, 1), k)] * sd(j, 1)) +
+                      (double)(bz[at(i, j, up(k, 2))] * su(k, 2)) - (double)(bz[at(i, j, down(k, 2))] * sd(k, 2));
+    m = fmax(m, fabs(db));
+  }
+  m = block_reduce_max(m);
+  if (threadIdx.x == 0) atomicMax(out_bits, (unsigned long long)__double_as_longlong(m * inv2dx));
+}
+
 // max face divergence of a CT face field, FP64 (ct.jl:176-185)
 static __global__ void __launch_bounds__(AUX_THREADS) divb_face_kernel(const float* __restrict__ bxf,
                                                                 const float* __restrict__ byf,
                                                                 const float* __restrict__ bzf, int nx, int ny,
-                                                                int nz, Cols cols, double invdx,
+                                                                int nz, int zc, double invdx,
                                                                 unsigned long long* out_bits) {
-  const int i = col_x(cols), j = col_y(cols);
+  const int i = blockIdx.x * COL_X + (threadIdx.x & 31), j = blockIdx.y * COL_Y + (threadIdx.x >> 5);
   double m = 0.0;
   if (i < nx && j < ny) {
-    const int z0 = blockIdx.z * cols.zc, z1 = min(z0 + cols.zc, nz);
+    const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
     const size_t nxy = (size_t)nx * ny, o = (size_t)j * nx + i;
     const size_t oip = (size_t)j * nx + wrap_inc(i, nx), ojp = (size_t)wrap_inc(j, ny) * nx + i;
     float z = bzf[z0 * nxy + o];
@@ -200,6 +230,24 @@ static __global__ void __launch_bounds__(AUX_THREADS) divb_face_kernel(const flo
       m = fmax(m, fabs(d));
       z = zp;
     }
+  }
+  m = block_reduce_max(m);
+  if (threadIdx.x == 0) atomicMax(out_bits, (unsigned long long)__double_as_longlong(m));
+}
+
+static __global__ void __launch_bounds__(AUX_THREADS) divb_face_flat_kernel(const float* __restrict__ bxf,
+                                                                     const float* __restrict__ byf,
+                                                                     const float* __restrict__ bzf, int nx, int ny,
+                                                                     int nz, double invdx,
+                                                                     unsigned long long* out_bits) {
+  const unsigned nc = (unsigned)nx * ny * nz, step = gridDim.x * blockDim.x;
+  double m = 0.0;
+  for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += step) {
+    const int q = c / (unsigned)nx, i = c - q * nx, k = q / ny, j = q - k * ny;
+    auto at = [&](int a, int b, int d) { return (d * ny + b) * nx + a; };
+    const double d = (((double)bxf[at(wrap_inc(i, nx), j, k)] - bxf[c]) + ((double)byf[at(i, wrap_inc(j, ny), k)] - byf[c]) +
+                      ((double)bzf[at(i, j, wrap_inc(k, nz))] - bzf[c])) * invdx;
+    m = fmax(m, fabs(d));
   }
   m = block_reduce_max(m);
   if (threadIdx.x == 0) atomicMax(out_bits, (unsigned long long)__double_as_longlong(m));

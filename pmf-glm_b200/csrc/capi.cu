@@ -726,15 +726,20 @@ int pmfmhd_max_divb(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* const U[9]
   if (!nonnull(U, 9)) return PMFMHD_EINVAL;
   cudaStream_t s = as_stream(stream);
   PMF_CK(cudaMemsetAsync(c->d_u64, 0, sizeof(unsigned long long), s));
-  // four cells per lane where rows and fields are 16-byte aligned and a tile's 128 columns are not
-  // mostly empty
-  bool v4 = g->nx % 4 == 0 && g->nx >= 64;
+  // by columns where those pay, four cells per lane where rows and fields are 16-byte aligned too
+  bool v4 = g->nx % 4 == 0 && cols_pay(g->nx / 4, g->ny, g->nz);
   for (int f = 5; f < 8; ++f) v4 = v4 && reinterpret_cast<uintptr_t>(U[f]) % 16 == 0;
-  Cols cols;
-  const dim3 tiles = col_grid(v4 ? g->nx / 4 : g->nx, g->ny, g->nz, c->sms, &cols);
-  const auto kernel = v4 ? divb4_kernel : divb_kernel;
-  kernel<<<tiles, AUX_THREADS, 0, s>>>(U[5], U[6], U[7], g->nx, g->ny, g->nz, cols, g->bc[0], g->bc[1], g->bc[2],
-                                       1.0 / (2.0 * (double)g->dx), c->d_u64);
+  const double inv2dx = 1.0 / (2.0 * (double)g->dx);
+  if (v4 || cols_pay(g->nx, g->ny, g->nz)) {
+    int zc;
+    const dim3 tiles = col_grid(v4 ? g->nx / 4 : g->nx, g->ny, g->nz, c->sms, &zc);
+    const auto kernel = v4 ? divb4_kernel : divb_kernel;
+    kernel<<<tiles, AUX_THREADS, 0, s>>>(U[5], U[6], U[7], g->nx, g->ny, g->nz, zc, g->bc[0], g->bc[1], g->bc[2], inv2dx,
+                                         2.0 * (double)g->dx * (1.0 - 1e-6), c->d_u64);
+  } else {
+    divb_flat_kernel<<<aux_blocks(c, ncells(g)), AUX_THREADS, 0, s>>>(U[5], U[6], U[7], g->nx, g->ny, g->nz, g->bc[0],
+                                                                     g->bc[1], g->bc[2], inv2dx, c->d_u64);
+  }
   PMF_CK(cudaGetLastError());
   PMF_CK(cudaMemcpyAsync(c->h_pin, c->d_u64, 8, cudaMemcpyDeviceToHost, s));
   PMF_CK(cudaStreamSynchronize(s));
@@ -749,10 +754,15 @@ int pmfmhd_max_divb_face(pmfmhd_ctx* c, const pmfmhd_grid* g, const float* ct, d
   cudaStream_t s = as_stream(stream);
   const long long nc = ncells(g);
   PMF_CK(cudaMemsetAsync(c->d_u64, 0, sizeof(unsigned long long), s));
-  Cols cols;
-  const dim3 tiles = col_grid(g->nx, g->ny, g->nz, c->sms, &cols);
-  divb_face_kernel<<<tiles, AUX_THREADS, 0, s>>>(ct, ct + nc, ct + 2 * nc, g->nx, g->ny, g->nz, cols,
-                                                 1.0 / (double)g->dx, c->d_u64);
+  if (cols_pay(g->nx, g->ny, g->nz)) {
+    int zc;
+    const dim3 tiles = col_grid(g->nx, g->ny, g->nz, c->sms, &zc);
+    divb_face_kernel<<<tiles, AUX_THREADS, 0, s>>>(ct, ct + nc, ct + 2 * nc, g->nx, g->ny, g->nz, zc,
+                                                   1.0 / (double)g->dx, c->d_u64);
+  } else {
+    divb_face_flat_kernel<<<aux_blocks(c, nc), AUX_THREADS, 0, s>>>(ct, ct + nc, ct + 2 * nc, g->nx, g->ny, g->nz,
+                                                                    1.0 / (double)g->dx, c->d_u64);
+  }
   PMF_CK(cudaGetLastError());
   PMF_CK(cudaMemcpyAsync(c->h_pin, c->d_u64, 8, cudaMemcpyDeviceToHost, s));
   PMF_CK(cudaStreamSynchronize(s));
