@@ -31,7 +31,13 @@ namespace {
 // chunk of z-planes. The wrapped x and y offsets of the stencil are formed once per column and
 // the values a plane shares with the next stay in registers, so a load costs one add. (With one
 // thread per cell and three integer remainders per neighbour the index arithmetic was most of
-// the work: a 128^3 CT subcycle took 473 us, 303 in this form.)
+// the work: a 128^3 CT subcycle took 473 us.) The loops over planes are unrolled by two (the next plane's
+// loads overlap this plane's arithmetic), and the order-4 stages hold four blocks an SM although they
+// spill some 100 bytes for it. Against plain loops with the compiler's own register counts:
+// order-4 induction 64^3 71 -> 57 us (GLM), 128^3 326 -> 283 (CT) and 221 -> 217 (GLM), 256^3 1.91 ->
+// 1.68 ms (CT); 128^3 force 22.9 -> 16.8 us. Indices wrap by selects: wrapped by loops, the lanes beyond
+// a small cube went round many times (8^3 GLM induction 43 us, 36 with selects, 40 with one thread per
+// cell).
 constexpr int kX = 32, kY = 8, kT = kX * kY;
 
 struct Cube {
@@ -55,19 +61,27 @@ struct Column {
   unsigned x[5], y[5];  // x[2 + d], y[2 + d]: wrapped x index and row offset at distance d
   int z0, z1;
   bool in;
+  // Periodic image of an index at most two outside: one conditional step reaches it unless N is 1. (The
+  // lanes beyond the cube take the last column's offsets, which they do not use.)
+  __device__ __forceinline__ static int wrap(int i, int n) {
+    const int r = i < 0 ? i + n : (i >= n ? i - n : i);
+    return n == 1 ? 0 : r;
+  }
   __device__ __forceinline__ explicit Column(const Cube& G) : N(G.N), nxy(G.N * G.N) {
-    const int i = blockIdx.x * kX + (threadIdx.x & (kX - 1)), j = blockIdx.y * kY + threadIdx.x / kX;
+    int i = blockIdx.x * kX + (threadIdx.x & (kX - 1)), j = blockIdx.y * kY + threadIdx.x / kX;
     in = i < N && j < N;
+    i = min(i, N - 1);
+    j = min(j, N - 1);
 #pragma unroll
     for (int d = -2; d <= 2; ++d) {
-      x[2 + d] = wrap_index(i + d, N);
-      y[2 + d] = wrap_index(j + d, N) * N;
+      x[2 + d] = wrap(i + d, N);
+      y[2 + d] = wrap(j + d, N) * N;
     }
     z0 = blockIdx.z * G.zc;
     z1 = min(z0 + G.zc, N);
   }
   __device__ __forceinline__ unsigned at(int dx, int dy) const { return y[2 + dy] + x[2 + dx]; }
-  __device__ __forceinline__ unsigned plane(int k) const { return (unsigned)(wrap_index(k, N) * nxy); }
+  __device__ __forceinline__ unsigned plane(int k) const { return (unsigned)(wrap(k, N) * nxy); }
 };
 
 struct F3 {
@@ -129,6 +143,7 @@ __global__ void __launch_bounds__(kT) force_kernel(Field3 B, float* __restrict__
   if (!C.in) return;
   const unsigned o = C.at(0, 0);
   F3 zm = B[C.plane(C.z0 - 1) + o], z0 = B[C.plane(C.z0) + o];
+#pragma unroll 2
   for (int k = C.z0; k < C.z1; ++k) {
     const unsigned b = C.plane(k);
     const F3 zp = B[C.plane(k + 1) + o];
@@ -171,6 +186,7 @@ __global__ void __launch_bounds__(kT) cell_emf_kernel(const float* __restrict__ 
     n = C.plane(C.z0);
     F3 b0 = B[n + o];
     float r0 = rho[n + o];
+#pragma unroll 2
     for (int k = C.z0; k < C.z1; ++k) {
       const unsigned b = C.plane(k);
       n = C.plane(k + 1);
@@ -246,6 +262,9 @@ template <int ORDER> struct Dissip {
   }
 };
 
+// Resident blocks an SM asked of a stage kernel (order 2 needs no cap)
+template <int ORDER> constexpr int kStageBlocks = ORDER == 4 ? 4 : 1;
+
 struct Stage {
   float dt, inv2dx, invdx, invdx2, eta;
 };
@@ -253,7 +272,7 @@ struct Stage {
 // GLM SSPRK2 stage (terminal_ct.jl:240-293). STAGE 0: out = B + dt*rhs(e, B).
 // STAGE 1: B <- (B + pB + dt*rhs(e, pB))/2 in place, E follows the magnetic energy.
 template <int ORDER, int STAGE>
-__global__ void __launch_bounds__(kT) glm_stage_kernel(Field3 e, float* bx, float* by, float* bz, float* pbx,
+__global__ void __launch_bounds__(kT, kStageBlocks<ORDER>) glm_stage_kernel(Field3 e, float* bx, float* by, float* bz, float* pbx,
                                                        float* pby, float* pbz, float* __restrict__ E, Cube G,
                                                        Stage S) {
   const Column C(G);
@@ -264,6 +283,7 @@ __global__ void __launch_bounds__(kT) glm_stage_kernel(Field3 e, float* bx, floa
   float exm = e.x[n + o], eym = e.y[n + o];
   n = C.plane(C.z0);
   float ex0 = e.x[n + o], ey0 = e.y[n + o];
+#pragma unroll 2
   for (int k = C.z0; k < C.z1; ++k) {
     const unsigned b = C.plane(k);
     n = C.plane(k + 1);
@@ -335,7 +355,7 @@ struct EdgeCurl {
 // CT SSPRK2 stage on the faces (terminal_ct.jl:347-407). STAGE 0: pf = f + dt*rate(e, f).
 // STAGE 1: f <- (f + pf + dt*rate(e, pf))/2 in place, Kahan-compensated when `comp`.
 template <int ORDER, int STAGE>
-__global__ void __launch_bounds__(kT) face_stage_kernel(Field3 ec, float* fx, float* fy, float* fz, float* pfx,
+__global__ void __launch_bounds__(kT, kStageBlocks<ORDER>) face_stage_kernel(Field3 ec, float* fx, float* fy, float* fz, float* pfx,
                                                         float* pfy, float* pfz, float* __restrict__ rbx,
                                                         float* __restrict__ rby, float* __restrict__ rbz, Cube G,
                                                         Stage S, int comp) {
@@ -344,6 +364,7 @@ __global__ void __launch_bounds__(kT) face_stage_kernel(Field3 ec, float* fx, fl
   const unsigned o = C.at(0, 0);
   Dissip<ORDER> dx(STAGE == 0 ? fx : pfx, C), dy(STAGE == 0 ? fy : pfy, C), dz(STAGE == 0 ? fz : pfz, C);
   EdgeCurl curl(ec, C);
+#pragma unroll 2
   for (int k = C.z0; k < C.z1; ++k) {
     const unsigned b = C.plane(k);
     const F3 u = curl(k, C);
@@ -381,6 +402,7 @@ __global__ void __launch_bounds__(kT) face_average_kernel(const float* __restric
   if (!C.in) return;
   const unsigned o = C.at(0, 0);
   float z0 = fz[C.plane(C.z0) + o];
+#pragma unroll 2
   for (int k = C.z0; k < C.z1; ++k) {
     const unsigned b = C.plane(k);
     const float zp = fz[C.plane(k + 1) + o];
@@ -412,6 +434,7 @@ __global__ void __launch_bounds__(kT) face_euler_kernel(Field3 ec, float* fx, fl
   if (!C.in) return;
   const unsigned o = C.at(0, 0);
   EdgeCurl curl(ec, C);
+#pragma unroll 2
   for (int k = C.z0; k < C.z1; ++k) {
     const unsigned b = C.plane(k);
     const F3 u = curl(k, C);
