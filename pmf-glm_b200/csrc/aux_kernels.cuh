@@ -65,7 +65,7 @@ inline dim3 col_grid(int nx, int ny, int nz, int sms, int* zc) {
   return dim3(tx, ty, (nz + *zc - 1) / *zc);
 }
 // Where columns pay: tiles at least half full (a 1 x 600 x 600 box took 67 us by columns and takes 31
-// with one thread per cell, 8 x 512 x 512 55 and 43), within what grid dimensions y and z can count.
+// with one thread per cell, 8 x 512 x 512 55 and 31), within what grid dimensions y and z can count.
 inline bool cols_pay(int nx, int ny, int nz) {
   const long long tx = (nx + COL_X - 1) / COL_X, ty = (ny + COL_Y - 1) / COL_Y;
   return 2LL * nx * ny >= tx * ty * AUX_THREADS && ty <= 65535 && nz <= 65535LL * COL_Z;
